@@ -10,6 +10,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
@@ -17,7 +18,7 @@ CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libfvedg_b200.so")
 OBJ = os.path.join(PKG, "_build")
 HOST_SRCS = ["host_mesh.cpp", "host_tables.cpp", "host_partition.cpp"]
-CUDA_SRCS = ["dg_api.cu"]
+CUDA_SRCS = ["dg_api.cu", "dg_mixed16.cu"]
 GENCODE = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CXX = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
 
@@ -54,6 +55,7 @@ def build(force=False, verbose_ptxas=False):
             _run([CXX, "-std=c++17", "-O3", "-mavx2", "-mfma", "-ffp-contract=fast", "-fPIC", "-Wall"] + inc + ["-c", s, "-o", o])
         objs.append(o)
     nvcc = _nvcc()
+    jobs = []
     for src in CUDA_SRCS:
         s = os.path.join(CSRC, src)
         o = os.path.join(OBJ, src + ".o")
@@ -61,8 +63,10 @@ def build(force=False, verbose_ptxas=False):
             cmd = [nvcc, "-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-ccbin", CXX] + GENCODE + inc
             if verbose_ptxas:
                 cmd.append("-Xptxas=-v")
-            _run(cmd + ["-c", s, "-o", o])
+            jobs.append(cmd + ["-c", s, "-o", o])
         objs.append(o)
+    with ThreadPoolExecutor(max_workers=max(1, len(jobs))) as pool:  # the CUDA sources side by side
+        list(pool.map(_run, jobs))
     if force or _stale(LIB, objs):
         _run([nvcc, "-shared", "-ccbin", CXX] + GENCODE + ["-o", LIB] + objs + ["-lcudart"])
     return LIB

@@ -13,7 +13,7 @@
 
 #include "dg_internal.h"
 #include "dg_kernels_fp64.cuh"
-#include "dg_kernels_mixed.cuh"
+#include "dg_mixed_host.cuh"
 #include "dg_kernels_fp64_tc.cuh"
 #include "dg_persistent.cuh"
 #include "dg_limiter.cuh"
@@ -950,7 +950,7 @@ int autotune_two_launch(dg_ctx* c, double dt, double* save, size_t nstate, char*
         cudaEventElapsedTime(&ms, e0, e1);
         ms *= 0.5f;
         js += std::string(i ? ", " : "") + "{\"element_kernel\": \"" + name(shapes[i]) + "\", \"warps_per_cta\": " +
-              std::to_string(shapes[i].warps) + ", \"elements_per_cta\": " + std::to_string(3 * shapes[i].warps) +
+              std::to_string(shapes[i].warps) + ", \"elements_per_cta\": " + std::to_string(shapes[i].group * shapes[i].warps) +
               ", \"ctas_per_sm\": " + std::to_string(shapes[i].ctas) + ", \"ms_per_step\": " + std::to_string(ms) + "}";
         if (rc == DG_OK && ms < best) { best = ms; bi = i; }
     }
@@ -958,7 +958,7 @@ int autotune_two_launch(dg_ctx* c, double dt, double* save, size_t nstate, char*
     c->mixed.elem_ctas = bi >= 0 ? shapes[bi].ctas : keep_c;
     js += "], \"chosen\": ";
     js += bi >= 0 ? "{\"element_kernel\": \"" + name(shapes[bi]) + "\", \"elements_per_cta\": " +
-                        std::to_string(3 * shapes[bi].warps) + ", \"ctas_per_sm\": " + std::to_string(shapes[bi].ctas) +
+                        std::to_string(shapes[bi].group * shapes[bi].warps) + ", \"ctas_per_sm\": " + std::to_string(shapes[bi].ctas) +
                         ", \"ms_per_step\": " + std::to_string(best) + "}}"
                   : std::string("null}");
     cudaMemcpyAsync(c->d_Un, save, nstate * sizeof(double), cudaMemcpyDeviceToDevice, c->stream);

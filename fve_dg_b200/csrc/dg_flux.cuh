@@ -298,6 +298,106 @@ __device__ __forceinline__ void lax_friedrichs_f32(const float UL[5], const floa
     Fh[4] = 0.5f * fmaf(lam, UL[4] - UR[4], fmaf(L.un, L.e, R.un * R.e));
 }
 
+// Two points at a time on the paired FP32 instructions (each lane of a pair is computed exactly as the
+// scalar forms above do, product by product). The pipe's rate is the same; half the instructions matter
+// where few warps are resident and issue or dependence latency is the limit.
+__device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.f), a); }
+__device__ __forceinline__ float2 rcp2(float2 a) { return make_float2(rcp_f32(a.x), rcp_f32(a.y)); }
+__device__ __forceinline__ float2 rsqrt2(float2 a) { return make_float2(rsqrtf(a.x), rsqrtf(a.y)); }
+__device__ __forceinline__ float2 max2(float2 a, float b) { return make_float2(fmaxf(a.x, b), fmaxf(a.y, b)); }
+__device__ __forceinline__ float2 abs2(float2 a) { return make_float2(fabsf(a.x), fabsf(a.y)); }
+__device__ __forceinline__ float2 dot2(const float2 a[3], const float n[3]) {
+    return fma2(a[2], f2(n[2]), fma2(a[1], f2(n[1]), mul2(a[0], f2(n[0]))));
+}
+
+struct StateF32x2 {
+    float2 r, ir, u[3], p, e, un, mn;
+};
+
+__device__ __forceinline__ StateF32x2 state_f32x2(const float2 U[5], const float n[3], float gm1) {
+    StateF32x2 s;
+    s.r = max2(U[0], 1e-16f);
+    s.ir = rcp2(s.r);
+    #pragma unroll
+    for (int i = 0; i < 3; ++i) s.u[i] = mul2(U[1 + i], s.ir);
+    const float2 k = fma2(s.u[2], U[3], fma2(s.u[1], U[2], mul2(s.u[0], U[1])));  // rho |u|^2
+    s.p = mul2(f2(gm1), fma2(f2(-0.5f), k, U[4]));
+    s.e = add2(U[4], s.p);
+    s.mn = dot2(U + 1, n);
+    s.un = mul2(s.mn, s.ir);
+    return s;
+}
+
+__device__ __forceinline__ void roe_f32x2(const float2 UL[5], const float2 UR[5], const float n[3], float gam, float2 Fh[5]) {
+    const float gm1 = gam - 1.f;
+    const StateF32x2 L = state_f32x2(UL, n, gm1), R = state_f32x2(UR, n, gm1);
+    const float2 sL = mul2(L.r, rsqrt2(L.r)), sR = mul2(R.r, rsqrt2(R.r));  // sqrt(rho)
+    const float2 iden = rcp2(add2(sL, sR));
+    const float2 wL = mul2(sL, iden), wR = mul2(sR, iden);
+    float2 ut[3];
+    #pragma unroll
+    for (int i = 0; i < 3; ++i) ut[i] = fma2(wL, L.u[i], mul2(wR, R.u[i]));
+    const float2 Ht = fma2(wL, mul2(L.e, L.ir), mul2(wR, mul2(R.e, R.ir)));
+    const float2 q2 = fma2(ut[2], ut[2], fma2(ut[1], ut[1], mul2(ut[0], ut[0])));
+    const float2 c2 = max2(mul2(f2(gm1), fma2(f2(-0.5f), q2, Ht)), 1e-16f);
+    const float2 qc = rsqrt2(c2);
+    const float2 ct = mul2(c2, qc), ic2 = mul2(qc, qc);
+    const float2 rt = mul2(sL, sR);
+    const float2 unt = dot2(ut, n);
+    const float2 dr = sub2(R.r, L.r), dp = sub2(R.p, L.p), dun = sub2(R.un, L.un);
+    float2 l1 = abs2(sub2(unt, ct)), l5 = abs2(add2(unt, ct));
+    const float2 l2 = abs2(unt);
+    const float2 delta = mul2(f2(0.1f), ct), d2 = mul2(delta, delta);
+    const float2 ihd = make_float2(__fdividef(0.5f, delta.x), __fdividef(0.5f, delta.y));
+    const float2 m1 = mul2(fma2(l1, l1, d2), ihd), m5 = mul2(fma2(l5, l5, d2), ihd);  // Harten's fix
+    l1.x = l1.x < delta.x ? m1.x : l1.x;
+    l1.y = l1.y < delta.y ? m1.y : l1.y;
+    l5.x = l5.x < delta.x ? m5.x : l5.x;
+    l5.y = l5.y < delta.y ? m5.y : l5.y;
+    const float2 rcd = mul2(mul2(rt, ct), dun), h2 = mul2(f2(0.5f), ic2);
+    const float2 w1 = mul2(l1, mul2(sub2(dp, rcd), h2)), w5 = mul2(l5, mul2(add2(dp, rcd), h2));
+    const float2 w2 = mul2(l2, sub2(dr, mul2(dp, ic2)));
+    const float2 W = add2(add2(w1, w2), w5), cw = mul2(ct, sub2(w5, w1)), lrt = mul2(l2, rt);
+    // Fh = (F_L + F_R - D) / 2 with D subtracted through its negated factors
+    const float2 nW = mul2(W, f2(-1.f)), ncw = mul2(cw, f2(-1.f)), nlrt = mul2(lrt, f2(-1.f));
+    const float2 ps = add2(L.p, R.p), half = f2(0.5f);
+    float2 uds = f2(0.f);
+    Fh[0] = mul2(half, add2(add2(L.mn, R.mn), nW));
+    #pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const float2 ni = f2(n[i]);
+        const float2 sh = fma2(dun, f2(-n[i]), sub2(R.u[i], L.u[i]));
+        uds = fma2(ut[i], sh, uds);
+        const float2 nD = fma2(nW, ut[i], fma2(ncw, ni, mul2(nlrt, sh)));
+        Fh[1 + i] = mul2(half, add2(fma2(UL[1 + i], L.un, fma2(UR[1 + i], R.un, mul2(ps, ni))), nD));
+    }
+    const float2 D4 = fma2(add2(w1, w5), Ht, fma2(cw, unt, fma2(mul2(half, w2), q2, mul2(lrt, uds))));
+    Fh[4] = mul2(half, sub2(fma2(L.un, L.e, mul2(R.un, R.e)), D4));
+}
+
+__device__ __forceinline__ void lax_friedrichs_f32x2(const float2 UL[5], const float2 UR[5], const float n[3], float gam,
+                                                     float2 Fh[5]) {
+    const StateF32x2 L = state_f32x2(UL, n, gam - 1.f), R = state_f32x2(UR, n, gam - 1.f);
+    auto speed = [&](const StateF32x2& s) {
+        const float2 v2 = fma2(s.u[2], s.u[2], fma2(s.u[1], s.u[1], mul2(s.u[0], s.u[0])));
+        const float2 c2 = max2(mul2(f2(gam), max2(mul2(s.p, s.ir), 1e-16f)), 1e-16f);
+        const float2 v = make_float2(v2.x > 0.f ? v2.x * rsqrtf(v2.x) : 0.f, v2.y > 0.f ? v2.y * rsqrtf(v2.y) : 0.f);
+        return fma2(c2, rsqrt2(c2), v);
+    };
+    const float2 a = speed(L), b = speed(R), lam = make_float2(fmaxf(a.x, b.x), fmaxf(a.y, b.y)), half = f2(0.5f);
+    const float2 ps = add2(L.p, R.p);
+    Fh[0] = mul2(half, fma2(lam, sub2(UL[0], UR[0]), add2(L.mn, R.mn)));
+    #pragma unroll
+    for (int i = 0; i < 3; ++i)
+        Fh[1 + i] = mul2(half, fma2(lam, sub2(UL[1 + i], UR[1 + i]),
+                                    fma2(UL[1 + i], L.un, fma2(UR[1 + i], R.un, mul2(ps, f2(n[i]))))));
+    Fh[4] = mul2(half, fma2(lam, sub2(UL[4], UR[4]), fma2(L.un, L.e, mul2(R.un, R.e))));
+}
+
 // Full 5 x 3 flux in FP32 (row = variable, column = direction), momenta used directly.
 __device__ __forceinline__ void flux_f32(const float U[5], float gm1, float F[5][3]) {
     const float r = fmaxf(U[0], 1e-16f), ir = rcp_f32(r);

@@ -26,7 +26,7 @@
 
 #include "dg_flux.cuh"
 #include "dg_kernels_fp64.cuh"
-#include "dg_kernels_mixed.cuh"
+#include "dg_mixed_host.cuh"
 
 namespace fvedg {
 

@@ -1,4 +1,5 @@
-// Mixed-precision form of the explicit DG operator.
+// Mixed-precision form of the explicit DG operator, groups of three: meshes too small to fill the SMs with
+// groups of sixteen (dg_kernels_mixed16.cuh, wide_groups in dg_mixed_host.cuh), and the helpers of both.
 //
 // The four dense contractions of a stage run on the tensor cores as BF16 MMAs with FP32
 // accumulation (mma.sync m16n8k16, plus an m16n8k8 tail so every K is padded to 8, not 16). Both
@@ -1044,409 +1045,6 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 3 : 6) element_mixed(
     const ElemBTabs bt{a.t.tva, a.t.tvp, a.t.tfl};
     for (int gi = blockIdx.x * WARPS + (threadIdx.x >> 5); gi < a.ngroups; gi += gridDim.x * WARPS)
         element_group_mixed<NB, NQV, NQF>(a, gi, sm, tabs, lane, bt);
-}
-
-// ------------------------------------------------------------------------------------------------
-// Host side
-// ------------------------------------------------------------------------------------------------
-struct MixedData {
-    bool ready = false;
-    int order = 0, qv = 0, qf = 0, nb = 0, nqv = 0, nqf = 0;
-    int64_t ncell = 0, nface = 0;
-    int nfgroups = 0, negroups = 0;
-    int nfgroups_inner = 0;  // face groups [0, nfgroups_inner) touch no ghost element
-    float gamma = 1.4f;
-    int flux = 0;
-    int sms = 148;
-    std::vector<void*> bufs;
-    MixedTables t{};
-    const FaceInfo* fi = nullptr;
-    const FaceGroup* fgroups = nullptr;
-    const ElemGroup* egroups = nullptr;
-    const double* geo = nullptr;
-    const double* inv_detj = nullptr;
-    const double* UD = nullptr;
-    uint32_t* dev = nullptr;          // face records [nface][face_rec_words(nqf)]
-    const double* dt_inst = nullptr;  // ensembles: per-instance dt (device), else null
-    const int* elem_inst = nullptr;
-    const double* Rv = nullptr;       // Navier-Stokes stepping: the stage input's viscous residual
-    int* err = nullptr;               // device status word of the mixed kernels (bounded waits)
-    // element kernel: 0 = loads phase by phase (8-warp CTAs, four per SM), 2 = each group's rows
-    // staged by TMA bulk copies (P1..P3, 16-byte aligned state buffers); chosen by dg_autotune
-    int elem_kernel = 0;
-    int elem_ctas = 1;                // resident CTAs per SM of the staged kernel: 1 or 2
-    // host copies the tile schedule of the persistent form is built from
-    std::vector<FaceGroup> hfg;
-    std::vector<ElemGroup> heg;
-    std::vector<int> hface_cells;  // [nface][2]
-};
-
-// X(order, qv, qf, NB, NQV, NQF, W): W warps per block of the element kernel
-#define FVEDG_MIXED_COMBOS(X)      \
-    X(1, 0, 1, 4, 4, 6, 8)         \
-    X(1, 0, 0, 4, 4, 4, 8)         \
-    X(1, 0, 2, 4, 4, 7, 8)         \
-    X(1, 2, 2, 4, 15, 7, 8)        \
-    X(2, 1, 2, 10, 11, 7, 8)       \
-    X(2, 1, 3, 10, 11, 24, 8)      \
-    X(2, 2, 3, 10, 15, 24, 8)      \
-    X(3, 3, 3, 20, 23, 24, 8)      \
-    X(3, 4, 3, 20, 31, 24, 8)      \
-    X(4, 5, 3, 35, 44, 24, 4)      \
-    X(4, 6, 3, 35, 57, 24, 4)
-
-inline bool mixed_supported(int order, int qv, int qf) {
-#define X(P, QV, QF, NB, NQV, NQF, W) \
-    if (order == P && qv == QV && qf == QF) return true;
-    FVEDG_MIXED_COMBOS(X)
-#undef X
-    return false;
-}
-
-template <typename T>
-inline int mixed_upload(MixedData& m, const T** dst, const std::vector<T>& v) {
-    void* p = nullptr;
-    if (cudaMalloc(&p, sizeof(T) * std::max<size_t>(v.size(), 1)) != cudaSuccess) return DG_E_NOMEM;
-    m.bufs.push_back(p);
-    if (!v.empty() && cudaMemcpy(p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-        return DG_E_CUDA;
-    *dst = (const T*)p;
-    return DG_OK;
-}
-
-template <typename T>
-inline int mixed_alloc(MixedData& m, T** dst, size_t n) {
-    void* p = nullptr;
-    if (cudaMalloc(&p, sizeof(T) * std::max<size_t>(n, 1)) != cudaSuccess) return DG_E_NOMEM;
-    m.bufs.push_back(p);
-    if (cudaMemset(p, 0, sizeof(T) * std::max<size_t>(n, 1)) != cudaSuccess) return DG_E_CUDA;
-    *dst = (T*)p;
-    return DG_OK;
-}
-
-// B operand of one contraction in fragment order. T is N x K row-major (N, K multiples of 8). Per
-// n-tile: for each full K tile, 32 lanes x {hi(c,c+1), hi(c+8,c+9), lo(c,c+1), lo(c+8,c+9)} of
-// row n = 8 nt + lane / 4, c = 16 t + 2 (lane % 4); then the tail, 32 lanes x {hi(c,c+1), lo(c,c+1)}.
-inline void append_frag_table(const std::vector<double>& T, int N, int K, std::vector<uint32_t>& out) {
-    const int n16 = K / 16;
-    const bool tail = (K % 16) != 0;
-    auto half = [&](int n, int k, bool lo) -> uint32_t {
-        const float f = (float)T[(size_t)n * K + k];
-        const __nv_bfloat16 h = __float2bfloat16_rn(f);
-        return (uint32_t)__bfloat16_as_ushort(lo ? __float2bfloat16_rn(f - __bfloat162float(h)) : h);
-    };
-    auto word = [&](int n, int c, bool lo) { return half(n, c, lo) | (half(n, c + 1, lo) << 16); };
-    for (int nt = 0; nt < N / 8; ++nt) {
-        for (int t = 0; t < n16; ++t)
-            for (int lane = 0; lane < 32; ++lane) {
-                const int n = nt * 8 + lane / 4, c = t * 16 + 2 * (lane % 4);
-                out.push_back(word(n, c, false));
-                out.push_back(word(n, c + 8, false));
-                out.push_back(word(n, c, true));
-                out.push_back(word(n, c + 8, true));
-            }
-        if (tail)
-            for (int lane = 0; lane < 32; ++lane) {
-                const int n = nt * 8 + lane / 4, c = n16 * 16 + 2 * (lane % 4);
-                out.push_back(word(n, c, false));
-                out.push_back(word(n, c, true));
-            }
-    }
-}
-
-// Faces with equal (perm0, perm1, kind) and elements with equal face maps (in canonical face
-// order: local face q is the one opposite local vertex q) are grouped in threes, in mesh order.
-// A partial group repeats its first member in the unused slots (never read as a row: rows of
-// unused slots are masked by the group size).
-// Face groups: faces of the same kind in threes, first the faces between owned elements, then
-// (from *nf_inner on) the faces touching a ghost element (cells >= ncell), whose fluxes need the
-// ghost rows of a halo exchange. Element groups: the owned elements [0, ncell).
-inline void build_groups(const std::vector<FaceInfo>& hfi, const std::vector<ElemFace>& hef, int64_t ncell,
-                         std::vector<FaceGroup>& fg, std::vector<ElemGroup>& eg, int* nf_inner) {
-    for (int halo = 0; halo < 2; ++halo) {
-        std::map<int64_t, FaceGroup> open_f;
-        for (int64_t f = 0; f < (int64_t)hfi.size(); ++f) {
-            const FaceInfo& F = hfi[f];
-            if ((F.c0 >= ncell || F.c1 >= ncell) != (halo == 1)) continue;
-            const int64_t key = (int64_t)(F.meta & 0xffffff) * 2 + (F.c1 >= 0 ? 1 : 0);
-            FaceGroup& g = open_f[key];
-            g.f[g.n++] = (int)f;
-            if (g.n == 3) { fg.push_back(g); g = FaceGroup{}; }
-        }
-        for (auto& kv : open_f)
-            if (kv.second.n > 0) {
-                for (int i = kv.second.n; i < 3; ++i) kv.second.f[i] = kv.second.f[0];
-                fg.push_back(kv.second);
-            }
-        if (halo == 0) *nf_inner = (int)fg.size();
-    }
-    std::map<std::vector<int>, ElemGroup> open_e;
-    for (int64_t e = 0; e < ncell; ++e) {
-        int face[4] = {-1, -1, -1, -1}, meta[4] = {0, 0, 0, 0};
-        for (int i = 0; i < 4; ++i) {
-            const ElemFace& ef = hef[4 * e + i];
-            const int p = ef.meta & 0xff;
-            const int q = 6 - kPermSlots[p][0] - kPermSlots[p][1] - kPermSlots[p][2];  // missing vertex
-            face[q] = ef.face;
-            meta[q] = ef.meta;
-        }
-        std::vector<int> key(meta, meta + 4);
-        ElemGroup& g = open_e[key];
-        g.e[g.n] = (int)e;
-        for (int q = 0; q < 4; ++q) { g.face[g.n][q] = face[q]; g.meta[q] = meta[q]; }
-        ++g.n;
-        if (g.n == 3) { eg.push_back(g); g = ElemGroup{}; }
-    }
-    for (auto& kv : open_e)
-        if (kv.second.n > 0) {
-            ElemGroup g = kv.second;
-            for (int i = g.n; i < 3; ++i) {
-                g.e[i] = g.e[0];
-                for (int q = 0; q < 4; ++q) g.face[i][q] = g.face[0][q];
-            }
-            eg.push_back(g);
-        }
-}
-
-inline int init_mixed(MixedData& m, const Tables& tab, const std::vector<double>& hgeo,
-                      const std::vector<FaceInfo>& hfi, const std::vector<ElemFace>& hef, int64_t ncell,
-                      int64_t nowned, int64_t nface, double gamma, int flux, int qv, int qf, const double* d_geo,
-                      const FaceInfo* d_fi, const ElemFace*, const double*) {
-    if (!mixed_supported(tab.order, qv, qf)) return DG_E_ARG;
-    const int NB = tab.nb, NQV = tab.nqv, NQF = tab.nqf;
-    const int KB = pad8(NB - 1), MF = pad8(NQF), MV = pad8(NQV), MJ = pad8(NB), KV = pad8(3 * NQV), KF = pad8(NQF);
-    m.order = tab.order; m.qv = qv; m.qf = qf; m.nb = NB; m.nqv = NQV; m.nqf = NQF;
-    m.ncell = ncell; m.nface = nface; m.gamma = (float)gamma; m.flux = flux;
-    std::vector<double> tva(MV * KB, 0.0), tvp(MJ * KV, 0.0);
-    std::vector<double> mv(NB * 3, 0.0), mf(24 * NB, 0.0), inv_mass(NB, 0.0), inv_detj(ncell, 0.0);
-    std::vector<uint32_t> ftfa, ftva, ftvp, ftfl;
-    for (int p = 0; p < 24; ++p) {
-        std::vector<double> tfa(MF * KB, 0.0), tfl(MJ * KF, 0.0);
-        for (int g = 0; g < NQF; ++g)
-            for (int b = 1; b < NB; ++b) tfa[g * KB + (b - 1)] = tab.phi_f[((size_t)p * NQF + g) * NB + b];
-        for (int j = 0; j < NB; ++j)
-            for (int g = 0; g < NQF; ++g) {
-                const double v = tab.w_f[g] * tab.phi_f[((size_t)p * NQF + g) * NB + j];
-                tfl[j * KF + g] = v;
-                mf[p * NB + j] += v;
-            }
-        append_frag_table(tfa, MF, KB, ftfa);
-        append_frag_table(tfl, MJ, KF, ftfl);
-    }
-    for (int g = 0; g < NQV; ++g)
-        for (int b = 1; b < NB; ++b) tva[g * KB + (b - 1)] = tab.phi_v[g * NB + b];
-    for (int j = 0; j < NB; ++j)
-        for (int g = 0; g < NQV; ++g)
-            for (int d = 0; d < 3; ++d) {
-                const double v = tab.dphi_vw[(g * NB + j) * 3 + d];
-                tvp[j * KV + 3 * g + d] = v;
-                mv[j * 3 + d] += v;
-            }
-    append_frag_table(tva, MV, KB, ftva);
-    append_frag_table(tvp, MJ, KV, ftvp);
-    for (int j = 0; j < NB; ++j) inv_mass[j] = 1.0 / tab.mass_ref[j];
-    for (int64_t e = 0; e < ncell; ++e) inv_detj[e] = 1.0 / hgeo[10 * e + 9];
-    double wsum = 0.0;
-    for (int g = 0; g < NQF; ++g) wsum += tab.w_f[g];
-    m.t.wsum = wsum;
-    int rc;
-    if ((rc = mixed_upload(m, &m.t.tfa, ftfa)) || (rc = mixed_upload(m, &m.t.tva, ftva)) ||
-        (rc = mixed_upload(m, &m.t.tvp, ftvp)) || (rc = mixed_upload(m, &m.t.tfl, ftfl)))
-        return rc;
-    if ((rc = mixed_upload(m, &m.t.mv, mv)) || (rc = mixed_upload(m, &m.t.mf, mf)) ||
-        (rc = mixed_upload(m, &m.t.inv_mass, inv_mass)) ||
-        (rc = mixed_upload(m, &m.t.wf32, std::vector<float>(tab.w_f.begin(), tab.w_f.end()))) ||
-        (rc = mixed_upload(m, &m.inv_detj, inv_detj)))
-        return rc;
-    std::vector<FaceGroup> fg;
-    std::vector<ElemGroup> eg;
-    build_groups(hfi, hef, nowned, fg, eg, &m.nfgroups_inner);  // element groups: owned cells only
-    m.nfgroups = (int)fg.size();
-    m.negroups = (int)eg.size();
-    if ((rc = mixed_upload(m, &m.fgroups, fg)) || (rc = mixed_upload(m, &m.egroups, eg))) return rc;
-    m.hfg = fg;
-    m.heg = eg;
-    m.hface_cells.resize(2 * hfi.size());
-    for (size_t f = 0; f < hfi.size(); ++f) {
-        m.hface_cells[2 * f] = hfi[f].c0;
-        m.hface_cells[2 * f + 1] = hfi[f].c1;
-    }
-    // padding columns of the A rows stay zero: allocation clears them and no kernel writes them
-    if ((rc = mixed_alloc(m, &m.dev, (size_t)nface * face_rec_words(NQF)))) return rc;
-    if ((rc = mixed_alloc(m, &m.err, 1))) return rc;
-    m.fi = d_fi; m.geo = d_geo;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&m.sms, cudaDevAttrMultiProcessorCount, dev);
-    m.ready = true;
-    return DG_OK;
-}
-
-inline void free_mixed(MixedData& m) {
-    for (void* p : m.bufs) cudaFree(p);
-    m.bufs.clear();
-    m.ready = false;
-}
-
-inline void set_mixed_dirichlet(MixedData& m, const double* UD) { m.UD = UD; }
-
-inline MixedFaceArgs face_args(const MixedData& m, const double* U, int face_mask, int g0 = 0, int g1 = -1) {
-    MixedFaceArgs fa;
-    fa.U = U; fa.fi = m.fi; fa.groups = m.fgroups; fa.UD = m.UD; fa.dev = m.dev;
-    fa.t = m.t; fa.ngroups = m.nfgroups; fa.gamma = m.gamma; fa.flux = m.flux;
-    if (g1 >= 0) {  // face groups [g0, g1) only
-        fa.groups = m.fgroups + g0;
-        fa.ngroups = g1 - g0;
-    }
-    fa.faces_mask = face_mask;
-    return fa;
-}
-
-inline MixedElemArgs elem_args(const MixedData& m, const double* U, const double* U0, double* out, int mode,
-                               double dt, double a0, double a1, int with_volume) {
-    MixedElemArgs ea;
-    ea.U = U; ea.U0 = U0; ea.out = out;
-    ea.dev = m.dev; ea.geo = m.geo; ea.inv_detj = m.inv_detj; ea.groups = m.egroups;
-    ea.t = m.t; ea.ngroups = m.negroups; ea.gamma = m.gamma; ea.volume = with_volume;
-    ea.dt = dt; ea.a0 = a0; ea.a1 = a1; ea.mode = mode;
-    ea.dt_inst = mode == 1 ? m.dt_inst : nullptr; ea.elem_inst = m.elem_inst;
-    ea.Rv = mode == 1 ? m.Rv : nullptr;
-    ea.err = m.err;
-    return ea;
-}
-
-// Opt a kernel into `smem` bytes of dynamic shared memory once per device.
-template <class Kernel>
-inline int ensure_smem(Kernel k, size_t smem, unsigned long long& done_mask) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return DG_E_CUDA;
-    const unsigned long long bit = 1ull << (dev & 63);
-    if (done_mask & bit) return DG_OK;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return DG_E_CUDA;
-    done_mask |= bit;
-    return DG_OK;
-}
-
-// which: 0 = face fluxes, 1 = element kernel (volume + face integrals + update).
-template <int NB, int NQV, int NQF, int WE>
-inline int mixed_launch(MixedData& m, int which, const double* U, const double* U0, double* out, int mode,
-                        double dt, double a0, double a1, int face_mask, int with_volume, cudaStream_t s, int g0,
-                        int g1) {
-    if (which == 0) {
-        constexpr int W = 4;  // 4-warp CTAs: finer-grained scheduling than 8 at the same occupancy
-        const int n = g1 < 0 ? m.nfgroups : g1 - g0;
-        const int g = (int)std::min<int64_t>((n + W - 1) / W, (int64_t)m.sms * 64);
-        face_flux_mixed<NB, NQF, W><<<g, W * 32, 0, s>>>(face_args(m, U, face_mask, g0, g1));
-    } else if (m.elem_kernel == 2 && (5 * NB * 8) % 16 == 0 && ((uintptr_t)U & 15) == 0 &&
-               ((uintptr_t)U0 & 15) == 0) {
-        if constexpr ((5 * NB * 8) % 16 == 0) {
-            const auto ea = elem_args(m, U, U0, out, mode, dt, a0, a1, with_volume);
-            if (m.elem_ctas == 2) {
-                constexpr int W = elem_staged_warps<NB, NQV, NQF>(2);
-                constexpr size_t smem = elem_staged_warp_smem<NB, NQV, NQF>() * W;
-                static unsigned long long done = 0;
-                int rc = ensure_smem(element_mixed_staged<NB, NQV, NQF, W, 2>, smem, done);
-                if (rc) return rc;
-                const int g = (int)std::min<int64_t>((m.negroups + W - 1) / W, (int64_t)m.sms * 2);
-                element_mixed_staged<NB, NQV, NQF, W, 2><<<g, W * 32, smem, s>>>(ea);
-            } else {
-                constexpr int W = elem_staged_warps<NB, NQV, NQF>(1);
-                constexpr size_t smem = elem_staged_warp_smem<NB, NQV, NQF>() * W;
-                static unsigned long long done = 0;
-                int rc = ensure_smem(element_mixed_staged<NB, NQV, NQF, W, 1>, smem, done);
-                if (rc) return rc;
-                const int g = (int)std::min<int64_t>((m.negroups + W - 1) / W, (int64_t)m.sms);
-                element_mixed_staged<NB, NQV, NQF, W, 1><<<g, W * 32, smem, s>>>(ea);
-            }
-        }
-    } else {
-        constexpr size_t smem = sizeof(ElemMixedSmem<NB, NQV, NQF>) * WE;
-        static unsigned long long done = 0;
-        int rc = ensure_smem(element_mixed<NB, NQV, NQF, WE>, smem, done);
-        if (rc) return rc;
-        const int g = (int)std::min<int64_t>((m.negroups + WE - 1) / WE, (int64_t)m.sms * 32);
-        element_mixed<NB, NQV, NQF, WE><<<g, WE * 32, smem, s>>>(
-            elem_args(m, U, U0, out, mode, dt, a0, a1, with_volume));
-    }
-    return cuda_status(cudaGetLastError());
-}
-
-// Element-kernel shapes of the two-launch schedule that dg_autotune times: the kernel (0: loads
-// phase by phase, 2: rows staged by bulk copies), warps per CTA (three elements each) and resident
-// CTAs per SM. Returns how many apply to this order and rule pair.
-struct ElemShape {
-    int kernel, warps, ctas;
-};
-inline int mixed_elem_shapes(const MixedData& m, ElemShape out[3]) {
-#define X(P, QV, QF, NB, NQV, NQF, W)                                                 \
-    if (m.order == P && m.qv == QV && m.qf == QF) {                                   \
-        int n = 0;                                                                    \
-        out[n++] = ElemShape{0, W, W == 8 ? 3 : 6};                                   \
-        if ((5 * NB * 8) % 16 == 0) {                                                 \
-            out[n++] = ElemShape{2, elem_staged_warps<NB, NQV, NQF>(1), 1};           \
-            out[n++] = ElemShape{2, elem_staged_warps<NB, NQV, NQF>(2), 2};           \
-        }                                                                             \
-        return n;                                                                     \
-    }
-    FVEDG_MIXED_COMBOS(X)
-#undef X
-    return 0;
-}
-
-// Face launches (which 0) cover face groups [g0, g1) (g1 < 0: all of them).
-inline int mixed_kernel(MixedData& m, int which, const double* U, const double* U0, double* out, int mode,
-                        double dt, double a0, double a1, int face_mask, int with_volume, cudaStream_t s,
-                        std::atomic<int64_t>* launches, int g0 = 0, int g1 = -1) {
-    if (!m.ready) return DG_E_ARG;
-    if (which == 0 && g1 >= 0 && g1 <= g0) return DG_OK;  // an empty range: nothing to launch
-    ++*launches;
-#define X(P, QV, QF, NB, NQV, NQF, W)                                                                           \
-    if (m.order == P && m.qv == QV && m.qf == QF)                                                               \
-        return mixed_launch<NB, NQV, NQF, W>(m, which, U, U0, out, mode, dt, a0, a1, face_mask, with_volume, s, \
-                                             g0, g1);
-    FVEDG_MIXED_COMBOS(X)
-#undef X
-    return DG_E_ARG;
-}
-
-// One stage: face fluxes, then the element kernel.
-template <class Timed>
-inline int mixed_stage(MixedData& m, const double* U, const double* U0, double* out, int mode, double dt, double a0,
-                       double a1, int face_mask, int with_volume, cudaStream_t s, std::atomic<int64_t>* launches,
-                       Timed&& timed) {
-    auto K = [&](int which) {
-        return mixed_kernel(m, which, U, U0, out, mode, dt, a0, a1, face_mask, with_volume, s, launches);
-    };
-    const int rc = timed(0, [&] { return K(0); });
-    if (rc) return rc;
-    return timed(1, [&] { return K(1); });
-}
-
-inline int residual_mixed(MixedData& m, const double* U, double* R, int part, cudaStream_t s,
-                          std::atomic<int64_t>* launches) {
-    const int mask = part == 0 ? 3 : part == 1 ? 0 : part == 2 ? 1 : 2;
-    return mixed_stage(m, U, U, R, 0, 0.0, 0.0, 0.0, mask, part == 0 || part == 1, s, launches,
-                       [](int, auto&& fn) { return fn(); });
-}
-
-inline int mixed_launches_per_step(const MixedData&) { return 6; }
-
-// SSP-RK3 step; `timed(cls, fn)` runs fn (one launch) and may bracket it with timing events.
-// `post(in, out, st)` runs after every stage st (the limiter, or nothing). Stages st0..st1-1 only
-// (one stage at a time when a halo exchange runs between stages).
-template <class Timed, class Post>
-inline int step_mixed(MixedData& m, double* Un, double* Ua, double* Ub, double dt, cudaStream_t s,
-                      std::atomic<int64_t>* launches, Timed&& timed, Post&& post, int st0 = 0, int st1 = 3) {
-    const double A0[3] = {0.0, 0.75, 1.0 / 3.0};
-    const double A1[3] = {1.0, 0.25, 2.0 / 3.0};
-    const double* in[3] = {Un, Ua, Ub};
-    double* out[3] = {Ua, Ub, Un};
-    for (int st = st0; st < st1; ++st) {
-        int rc = mixed_stage(m, in[st], Un, out[st], 1, dt, A0[st], A1[st], 3, 1, s, launches, timed);
-        if (rc || (rc = post(in[st], out[st], st))) return rc;
-    }
-    return DG_OK;
 }
 
 }  // namespace fvedg

@@ -17,19 +17,10 @@
 // last CTA to leave re-arms the ticket and the completion counters for the next launch, so a CUDA
 // graph replays the three launches of a step as they are.
 #pragma once
-#include "dg_kernels_mixed.cuh"
+#include "dg_mixed_host.cuh"
+#include "dg_persistent.h"
 
 namespace fvedg {
-
-constexpr int kMaxRegions = 64;
-
-struct QueueState {
-    unsigned int ticket;              // next tile of the list
-    unsigned int exits;               // CTAs that have left this launch
-    int error;                        // DG_OK or DG_E_WATCHDOG
-    int pad;
-    unsigned int done[kMaxRegions];   // face groups completed, per region
-};
 
 constexpr long long kSpinLimit = 1ll << 24;  // about a second of 64 ns naps
 
@@ -65,9 +56,7 @@ __host__ __device__ constexpr size_t persistent_warp_smem() {
 #endif
 template <int NB, int NQV, int NQF, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? FVEDG_PERSIST_MINB8 : 6)
-    stage_persistent_mixed(MixedFaceArgs fa, MixedElemArgs ea, QueueState* q, const int4* __restrict__ tiles,
-                           int ntiles, const unsigned long long* __restrict__ deps,
-                           const unsigned int* __restrict__ total, long long spin_limit) {
+    stage_persistent_mixed(MixedFaceArgs fa, MixedElemArgs ea, TileQueue Q) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ ElemTables<NB> tabs;
     __shared__ int4 s_tile;
@@ -75,28 +64,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? FVEDG_PERSIST_MINB8 :
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned char* wsm = smem_raw + persistent_warp_smem<NB, NQV, NQF>() * warp;
     for (;;) {
-        if (threadIdx.x == 0) {
-            const unsigned int t = atomicAdd(&q->ticket, 1u);
-            int4 tl = t < (unsigned int)ntiles ? tiles[t] : make_int4(-1, 0, 0, 0);
-            if (tl.x == 1) {  // element tile: wait until the face regions it reads are complete
-                unsigned long long need = deps[tl.w];
-                while (need) {
-                    const int f = __ffsll((long long)need) - 1;
-                    const volatile unsigned int* d = &q->done[f];
-                    long long spins = 0;
-                    while (*d < total[f]) {
-                        __nanosleep(64);
-                        if (++spins > spin_limit) {
-                            atomicExch(&q->error, DG_E_WATCHDOG);
-                            break;
-                        }
-                    }
-                    need &= need - 1;
-                }
-                __threadfence();
-            }
-            s_tile = tl;
-        }
+        if (threadIdx.x == 0) s_tile = take_tile(Q);
         __syncthreads();
         const int4 tl = s_tile;
         if (tl.x < 0) break;
@@ -105,7 +73,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? FVEDG_PERSIST_MINB8 :
                 face_group_mixed<NB, NQF>(fa, gi, *reinterpret_cast<FaceMixedSmem<NQF>*>(wsm), lane);
             __threadfence();  // this CTA's face data is visible before the region count moves
             __syncthreads();
-            if (threadIdx.x == 0) atomicAdd(&q->done[tl.w], (unsigned int)(tl.z - tl.y));
+            if (threadIdx.x == 0) atomicAdd(&Q.q->done[tl.w], (unsigned int)(tl.z - tl.y));
         } else {
             auto& esm = *reinterpret_cast<ElemMixedSmem<NB, NQV, NQF>*>(wsm);
             const ElemBTabs bt{ea.t.tva, ea.t.tvp, ea.t.tfl};
@@ -113,36 +81,30 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? FVEDG_PERSIST_MINB8 :
             __syncthreads();
         }
     }
-    if (threadIdx.x == 0) {  // the last CTA out re-arms the queue
-        __threadfence();
-        if (atomicAdd(&q->exits, 1u) == gridDim.x - 1) {
-            q->ticket = 0u;
-            for (int r = 0; r < kMaxRegions; ++r) q->done[r] = 0u;
-            __threadfence();
-            q->exits = 0u;
-        }
-    }
+    if (threadIdx.x == 0) leave_queue(Q);
 }
 
 // Builds the tile list for `pp`: reorders the face groups by region (the face kernel of the
 // two-launch form does not depend on their order) and uploads the list. Synchronous: call outside
 // any stream capture (context creation, the autotuner).
-inline int build_schedule(MixedData& m, QueueSchedule& qs, const PersistentParams& pp) {
+template <class FG, class EG>
+inline int build_schedule_of(MixedData& m, std::vector<FG>& hfg, const std::vector<EG>& heg, const FG* fgroups,
+                             QueueSchedule& qs, const PersistentParams& pp, int tile_f, int tile_e) {
     const int ne = m.negroups, nf = m.nfgroups;
     if (ne < 1 || nf < 1) return DG_E_ARG;
     const int R = std::max(1, std::min({pp.regions, kMaxRegions, ne}));
-    const int tf = std::max(1, pp.tile_f), te = std::max(1, pp.tile_e), lag = std::max(0, pp.lag);
+    const int tf = std::max(1, tile_f), te = std::max(1, tile_e), lag = std::max(0, pp.lag);
     std::vector<int> ereg(m.ncell, R), greg(ne);  // ghost cells (in no element group) stay at R
     for (int g = 0; g < ne; ++g) {
         greg[g] = (int)((int64_t)g * R / ne);
-        for (int i = 0; i < m.heg[g].n; ++i) ereg[m.heg[g].e[i]] = greg[g];
+        for (int i = 0; i < heg[g].n; ++i) ereg[heg[g].e[i]] = greg[g];
     }
     // face groups by region (lowest region among their cells), stable within a region
     std::vector<int> freg(nf);
     for (int g = 0; g < nf; ++g) {
         int r = R;
-        for (int i = 0; i < m.hfg[g].n; ++i) {
-            const int f = m.hfg[g].f[i];
+        for (int i = 0; i < hfg[g].n; ++i) {
+            const int f = hfg[g].f[i];
             r = std::min(r, ereg[m.hface_cells[2 * f]]);
             if (m.hface_cells[2 * f + 1] >= 0) r = std::min(r, ereg[m.hface_cells[2 * f + 1]]);
         }
@@ -151,19 +113,19 @@ inline int build_schedule(MixedData& m, QueueSchedule& qs, const PersistentParam
     std::vector<int> order(nf);
     for (int g = 0; g < nf; ++g) order[g] = g;
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return freg[x] < freg[y]; });
-    std::vector<FaceGroup> fg(nf);
+    std::vector<FG> fg(nf);
     std::vector<int> fg_reg(nf), face_reg(m.nface, 0);
     std::vector<unsigned int> total(R, 0u);
     for (int i = 0; i < nf; ++i) {
-        fg[i] = m.hfg[order[i]];
+        fg[i] = hfg[order[i]];
         fg_reg[i] = freg[order[i]];
         ++total[fg_reg[i]];
         for (int k = 0; k < fg[i].n; ++k) face_reg[fg[i].f[k]] = fg_reg[i];
     }
     std::vector<unsigned long long> deps(R, 0ull);
     for (int g = 0; g < ne; ++g)
-        for (int i = 0; i < m.heg[g].n; ++i)
-            for (int q = 0; q < 4; ++q) deps[greg[g]] |= 1ull << face_reg[m.heg[g].face[i][q]];
+        for (int i = 0; i < heg[g].n; ++i)
+            for (int q = 0; q < 4; ++q) deps[greg[g]] |= 1ull << face_reg[heg[g].face[i][q]];
     // element region r goes after face region min(last dependency + lag, R - 1)
     std::vector<std::vector<int>> after(R);
     for (int r = 0; r < R; ++r) {
@@ -187,9 +149,9 @@ inline int build_schedule(MixedData& m, QueueSchedule& qs, const PersistentParam
                 tiles.push_back(make_int4(1, g, std::min(g + te, ebeg[r + 1]), r));
     }
     // upload: the reordered face groups into the existing buffer, the schedule into fresh ones
-    if (cudaMemcpy((void*)m.fgroups, fg.data(), sizeof(FaceGroup) * nf, cudaMemcpyHostToDevice) != cudaSuccess)
+    if (cudaMemcpy((void*)fgroups, fg.data(), sizeof(FG) * nf, cudaMemcpyHostToDevice) != cudaSuccess)
         return DG_E_CUDA;
-    m.hfg = fg;
+    hfg = fg;
     if (qs.tiles) cudaFree(qs.tiles);
     if (qs.deps) cudaFree(qs.deps);
     if (qs.total) cudaFree(qs.total);
@@ -210,11 +172,25 @@ inline int build_schedule(MixedData& m, QueueSchedule& qs, const PersistentParam
     return DG_OK;
 }
 
+// Tiles are given in groups of three; a context of groups of sixteen takes about as many items per face tile
+// and as many groups per element tile as per face tile, so that the CTA's warps have one or more each.
+inline int build_schedule(MixedData& m, QueueSchedule& qs, const PersistentParams& pp) {
+    if (m.wide) {
+        const int t = std::max(3, pp.tile_f * 3 / 8);
+        return build_schedule_of(m, m.hfg16, m.heg16, m.fgroups16, qs, pp, t, t);
+    }
+    return build_schedule_of(m, m.hfg, m.heg, m.fgroups, qs, pp, pp.tile_f, pp.tile_e);
+}
+
 inline void free_schedule(QueueSchedule& qs) {
     if (qs.tiles) cudaFree(qs.tiles);
     if (qs.deps) cudaFree(qs.deps);
     if (qs.total) cudaFree(qs.total);
     qs = QueueSchedule{};
+}
+
+inline TileQueue tile_queue(QueueState* q, const QueueSchedule& qs, const PersistentParams& pp) {
+    return TileQueue{q, qs.tiles, qs.ntiles, qs.deps, qs.total, pp.spin_limit > 0 ? pp.spin_limit : kSpinLimit};
 }
 
 template <int NB, int NQV, int NQF, int W = 8>
@@ -238,10 +214,8 @@ inline int persistent_launch(MixedData& m, QueueState* q, const QueueSchedule& q
         done |= 1ull << (dev & 63);
     }
     const int bps = pp.max_blocks > 0 ? std::min(per_sm[dev & 63], pp.max_blocks) : per_sm[dev & 63];
-    const MixedFaceArgs fa = face_args(m, U, face_mask);
-    const MixedElemArgs ea = elem_args(m, U, U0, out, mode, dt, a0, a1, with_volume);
-    kern<<<m.sms * bps, W * 32, smem, s>>>(fa, ea, q, qs.tiles, qs.ntiles, qs.deps, qs.total,
-                                           pp.spin_limit > 0 ? pp.spin_limit : kSpinLimit);
+    kern<<<m.sms * bps, W * 32, smem, s>>>(face_args(m, U, face_mask),
+                                           elem_args(m, U, U0, out, mode, dt, a0, a1, with_volume), tile_queue(q, qs, pp));
     return cuda_status(cudaGetLastError());
 }
 
@@ -250,6 +224,12 @@ inline int persistent_kernel(MixedData& m, QueueState* q, const QueueSchedule& q
                              int face_mask, int with_volume, cudaStream_t s, std::atomic<int64_t>* launches) {
     if (!m.ready) return DG_E_ARG;
     ++*launches;
+    if (m.wide) {
+        if (!qs.ready || !(qs.built == pp)) return DG_E_STATE;
+        return mixed16_stage(m.order, m.qv, m.qf, m.sms, face_args16(m, U, face_mask),
+                             elem_args16(m, U, U0, out, mode, dt, a0, a1, with_volume), tile_queue(q, qs, pp),
+                             pp.max_blocks, s);
+    }
 #define X(P, QV, QF, NB, NQV, NQF, W)                                                                              \
     if (m.order == P && m.qv == QV && m.qf == QF)                                                                  \
         return persistent_launch<NB, NQV, NQF, W>(m, q, qs, pp, U, U0, out, mode, dt, a0, a1, face_mask,           \
