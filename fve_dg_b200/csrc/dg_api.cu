@@ -15,6 +15,7 @@
 #include "dg_kernels_fp64.cuh"
 #include "dg_mixed_host.cuh"
 #include "dg_kernels_fp64_tc.cuh"
+#include "dg_fp64_rows_host.cuh"
 #include "dg_persistent.cuh"
 #include "dg_limiter.cuh"
 #include "dg_viscous.cuh"
@@ -76,6 +77,7 @@ struct dg_ctx {
     double* d_red_out = nullptr;
     MixedData mixed;               // mixed-precision form buffers
     TcData tc;                     // FP64 form on the FP64 tensor cores (the configurations' rules)
+    Rows8Data rows;                // the same in rows of eight (large meshes, and orders 0 and 5)
     bool have_state = false;
     bool has_dirichlet = false;    // some boundary face is Dirichlet: U_D must be set first
     cudaGraphExec_t graph = nullptr;
@@ -278,8 +280,31 @@ TcElemArgs tc_elem_args(dg_ctx* c, const double* U, const double* U0, double* ou
     return a;
 }
 
+Rows8FaceArgs rows8_face_args(dg_ctx* c, const double* U, int mask) {
+    Rows8FaceArgs a;
+    a.U = U; a.fi = c->d_fi; a.groups = c->rows.fgroups; a.ngroups = c->rows.nfgroups; a.UD = c->d_UD; a.rec = c->rows.rec;
+    a.t = c->rows.t; a.gamma = c->cfg.gamma; a.flux = c->cfg.flux; a.faces_mask = mask; a.err = c->rows.err;
+    return a;
+}
+
+Rows8ElemArgs rows8_elem_args(dg_ctx* c, const double* U, const double* U0, double* out, int mode, double dt, double a0,
+                              double a1, int with_volume) {
+    Rows8ElemArgs a;
+    a.U = U; a.U0 = U0; a.out = out; a.rec = c->rows.rec; a.jd = c->rows.jd; a.inv_detj = c->rows.inv_detj;
+    a.groups = c->rows.egroups; a.ngroups = c->rows.negroups; a.t = c->rows.t; a.gamma = c->cfg.gamma;
+    a.with_volume = with_volume; a.mode = mode; a.dt = dt; a.a0 = a0; a.a1 = a1;
+    a.dt_inst = mode == 1 ? c->d_dt_inst : nullptr; a.elem_inst = c->d_elem_inst;
+    a.Rv = (mode == 1 && c->cfg.mu > 0.0) ? c->d_Rv : nullptr;
+    a.err = c->rows.err;
+    return a;
+}
+
 // Face-flux launch of the FP64 form (tensor-core kernels where the rules have them).
 int fp64_face(dg_ctx* c, const double* U, int mask, cudaStream_t s) {
+    if (c->rows.ready) {
+        ++g_launches;
+        return rows8_face(c->rows.order, c->rows.qv, c->rows.qf, c->rows.sms, rows8_face_args(c, U, mask), s);
+    }
     if (c->tc.ready) {
         ++g_launches;
         return tc_kernel(c->tc, 0, tc_face_args(c, U, mask), TcElemArgs{}, s);
@@ -290,6 +315,11 @@ int fp64_face(dg_ctx* c, const double* U, int mask, cudaStream_t s) {
 // Element launch of the FP64 form: R (mode 0) or the RK stage out = a0 U0 + a1 (U + dt L) (mode 1).
 int fp64_element(dg_ctx* c, const double* U, const double* U0, double* out, int mode, double dt, double a0,
                  double a1, int with_volume, cudaStream_t s) {
+    if (c->rows.ready) {
+        ++g_launches;
+        return rows8_element(c->rows.order, c->rows.qv, c->rows.qf, c->rows.sms,
+                             rows8_elem_args(c, U, U0, out, mode, dt, a0, a1, with_volume), s);
+    }
     if (c->tc.ready) {
         ++g_launches;
         return tc_kernel(c->tc, 1, TcFaceArgs{}, tc_elem_args(c, U, U0, out, mode, dt, a0, a1, with_volume), s);
@@ -477,10 +507,11 @@ int launches_per_step(const dg_ctx* c) {
 // waits (DG_OK or DG_E_WATCHDOG); a set word is cleared.
 int check_queue(dg_ctx* c) {
     int err = 0;
-    if (c->mixed.err) {
-        if (cudaMemcpy(&err, c->mixed.err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return DG_E_CUDA;
+    for (int* word : {c->mixed.err, c->rows.err}) {
+        if (!word) continue;
+        if (cudaMemcpy(&err, word, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return DG_E_CUDA;
         if (err != DG_OK) {
-            cudaMemset(c->mixed.err, 0, sizeof(int));
+            cudaMemset(word, 0, sizeof(int));
             return DG_E_WATCHDOG;
         }
     }
@@ -520,6 +551,7 @@ void free_ctx(dg_ctx* c) {
     free_schedule(c->qs);
     free_mixed(c->mixed);
     free_tc(c->tc);
+    free_rows8(c->rows);
     if (c->d_queue) cudaFree(c->d_queue);
     if (c->d_dt_inst) cudaFree(c->d_dt_inst);
     if (c->d_lim_bnd) cudaFree(c->d_lim_bnd);
@@ -649,6 +681,15 @@ dg_ctx* create_impl(const dg_mesh_desc* mesh, const dg_config* cfg, int* err, co
         hh[e] = geo.detj[e] / 6.0 / area;
     }
     const size_t nstate = (size_t)c->ncell * 5 * nb;
+    {
+        int dev = 0, sms = 148;
+        if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
+            c->sms = sms;
+    }
+    std::vector<FaceGroup8> fg8;
+    std::vector<ElemGroup8> eg8;
+    const bool rows = cfg->precision == DG_PREC_FP64 &&
+                      rows8_groups(cfg->order, qv, qf, c->sms, hfi, hef, c->nowned, fg8, eg8);
     if ((rc = upload(&c->d_h, hh)) || (rc = upload(&c->d_dphi_v, c->tab.dphi_v)) ||
         (rc = upload(&c->d_dphi_f, c->tab.dphi_f)))
         return fail(c, rc);
@@ -657,7 +698,7 @@ dg_ctx* create_impl(const dg_mesh_desc* mesh, const dg_config* cfg, int* err, co
         (rc = upload(&c->d_w_v, c->tab.w_v)) || (rc = upload(&c->d_phi_f, c->tab.phi_f)) ||
         (rc = upload(&c->d_phi_fT, c->tab.phi_fT)) || (rc = upload(&c->d_phi_vT, c->tab.phi_vT)) ||
         (rc = upload(&c->d_w_f, c->tab.w_f)) || (rc = upload(&c->d_mass_ref, c->tab.mass_ref)) ||
-        (rc = dev_alloc(&c->d_Fh, (cfg->precision == DG_PREC_FP64 && !tc_supported(cfg->order, qv, qf))
+        (rc = dev_alloc(&c->d_Fh, (cfg->precision == DG_PREC_FP64 && !rows && !tc_supported(cfg->order, qv, qf))
                                       ? (size_t)c->nface * nqf * 5 : 0)) ||
         (rc = dev_alloc(&c->d_Un, nstate)) ||
         (rc = dev_alloc(&c->d_Ua, nstate)) || (rc = dev_alloc(&c->d_Ub, nstate)) ||
@@ -672,7 +713,10 @@ dg_ctx* create_impl(const dg_mesh_desc* mesh, const dg_config* cfg, int* err, co
         std::vector<double> dts(c->ninst, 0.0);
         if ((rc = upload(&c->d_elem_inst, inst)) || (rc = upload(&c->d_dt_inst, dts))) return fail(c, rc);
     }
-    if (cfg->precision == DG_PREC_FP64 && tc_supported(cfg->order, qv, qf)) {
+    if (rows) {
+        c->rows.sms = c->sms;
+        if ((rc = init_rows8(c->rows, c->tab, hgeo, fg8, eg8, c->ncell, c->nface, qv, qf))) return fail(c, rc);
+    } else if (cfg->precision == DG_PREC_FP64 && tc_supported(cfg->order, qv, qf)) {
         if ((rc = init_tc(c->tc, c->tab, hgeo, hfi, hef, c->ncell, c->nowned, c->nface, qv, qf))) return fail(c, rc);
     }
     if (cfg->precision == DG_PREC_MIXED) {
@@ -688,11 +732,6 @@ dg_ctx* create_impl(const dg_mesh_desc* mesh, const dg_config* cfg, int* err, co
         // the faces between owned elements first (dg_ssprk3_stage_phase)
         if (cfg->schedule == 1 || c->nowned == c->ncell)
             if ((rc = build_schedule(c->mixed, c->qs, c->pp))) return fail(c, rc);
-    }
-    {
-        int dev = 0, sms = 148;
-        if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
-            c->sms = sms;
     }
     // Navier-Stokes stepping: the viscous buffers now, so that no step allocates (graph capture)
     if (cfg->mu > 0.0) {

@@ -1,0 +1,140 @@
+// Host side of the FP64 kernels for rows of eight: tables in fragment order, groups and buffers.
+#pragma once
+#include <vector>
+
+#include "dg_fp64_rows.h"
+#include "dg_mixed_host.cuh"
+
+namespace fvedg {
+
+struct Rows8Data {
+    bool ready = false;
+    int order = 0, qv = 0, qf = 0;
+    int nfgroups = 0, negroups = 0;
+    int sms = 148;
+    std::vector<void*> bufs;
+    Rows8Tables t{};
+    const FaceGroup8* fgroups = nullptr;
+    const ElemGroup8* egroups = nullptr;
+    const double* jd = nullptr;
+    const double* inv_detj = nullptr;
+    double* rec = nullptr;  // [nface][5][moment_row(nb)]
+    int* err = nullptr;
+};
+
+inline bool rows8_supported(int order, int qv, int qf) {
+#define X(P, QV, QF, NB, NQV, NQF) \
+    if (order == P && qv == QV && qf == QF) return true;
+    FVEDG_ROWS8_COMBOS(X)
+#undef X
+    return false;
+}
+
+template <typename T>
+inline int rows8_upload(Rows8Data& m, const T** dst, const std::vector<T>& v) {
+    void* p = nullptr;
+    if (cudaMalloc(&p, sizeof(T) * std::max<size_t>(v.size(), 1)) != cudaSuccess) return DG_E_NOMEM;
+    m.bufs.push_back(p);
+    if (!v.empty() && cudaMemcpy(p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+        return DG_E_CUDA;
+    *dst = (const T*)p;
+    return DG_OK;
+}
+
+// Whether a mesh runs in rows of eight, with its groups. Orders 0 and 5 have no other tensor-core kernels and
+// always do (P0 56 -> 39 us a step at n = 4 against the runtime-size kernels, P5 326 -> 233; n = 24: 372 -> 260 and
+// 16,345 -> 4,838). For the others groups of three are the faster on small meshes, where a warp's chain of work
+// decides (us a step, three / eight: P1 29 / 34 at n = 4, 31 / 34 at n = 8, 44 / 44 at n = 11, 76 / 71 at n = 14; P2
+// 43 / 46, 62 / 65, 109 / 108 from n = 8; P3 78 / 75, 125 / 118, 231 / 206; P4 115 / 122, 252 / 192, 451 / 372): five
+// groups per SM, about 6,000 cells. And the groups must be reasonably full (many classes of face maps leave as many
+// partial groups).
+inline bool rows8_groups(int order, int qv, int qf, int sms, const std::vector<FaceInfo>& hfi,
+                         const std::vector<ElemFace>& hef, int64_t nowned, std::vector<FaceGroup8>& fg,
+                         std::vector<ElemGroup8>& eg) {
+    if (!rows8_supported(order, qv, qf)) return false;
+    if (order >= 1 && order <= 4 && nowned < (int64_t)5 * kRows8 * sms) return false;
+    int inner = 0;
+    build_groups(hfi, hef, nowned, fg, eg, &inner);
+    return (int64_t)eg.size() * kRows8 * 3 <= nowned * 4 && (int64_t)fg.size() * kRows8 * 3 <= (int64_t)hfi.size() * 4;
+}
+
+inline int init_rows8(Rows8Data& m, const Tables& tab, const std::vector<double>& hgeo, const std::vector<FaceGroup8>& fg,
+                      const std::vector<ElemGroup8>& eg, int64_t ncell, int64_t nface, int qv, int qf) {
+    const int NB = tab.nb, NQV = tab.nqv, NQF = tab.nqf, NM = face_moments(NB), MR = moment_row(NB);
+    const int KT = (NB + 3) / 4, NF = pad8(NQF) / 8, NV = pad8(NQV) / 8, NJ = pad8(NB) / 8, MT = (MR + 7) / 8;
+    const int KF = moment_ktiles(NB);
+    m.order = tab.order; m.qv = qv; m.qf = qf;
+    std::vector<double> psi, norm, T, tf, tm, tv, tw, tl;
+    face_moment_basis(tab.order, qf, psi, norm);
+    face_moment_maps(tab, qf, psi, norm, T);
+    for (int p = 0; p < 24; ++p)
+        for (int nt = 0; nt < NF; ++nt)
+            for (int kt = 0; kt < KT; ++kt)
+                for (int l = 0; l < 32; ++l) {
+                    const int g = 8 * nt + l / 4, b = 4 * kt + l % 4;
+                    tf.push_back(g < NQF && b < NB ? tab.phi_f[((size_t)p * NQF + g) * NB + b] : 0.0);
+                }
+    for (int nt = 0; nt < NF; ++nt)
+        for (int i = 0; i < 2; ++i)
+            for (int mt = 0; mt < MT; ++mt)
+                for (int l = 0; l < 32; ++l) {
+                    const int g = 8 * nt + 2 * (l % 4) + i, k = 8 * mt + l / 4;
+                    tm.push_back(g < NQF && k < NM ? tab.w_f[g] * psi[(size_t)k * NQF + g] : 0.0);
+                }
+    for (int nt = 0; nt < NV; ++nt)
+        for (int kt = 0; kt < KT; ++kt)
+            for (int l = 0; l < 32; ++l) {
+                const int g = 8 * nt + l / 4, b = 4 * kt + l % 4;
+                tv.push_back(g < NQV && b < NB ? tab.phi_v[(size_t)g * NB + b] : 0.0);
+            }
+    for (int nt = 0; nt < NV; ++nt)
+        for (int d = 0; d < 3; ++d)
+            for (int i = 0; i < 2; ++i)
+                for (int j = 0; j < NJ; ++j)
+                    for (int l = 0; l < 32; ++l) {
+                        const int g = 8 * nt + 2 * (l % 4) + i, b = 8 * j + l / 4;
+                        tw.push_back(g < NQV && b < NB ? tab.dphi_vw[((size_t)g * NB + b) * 3 + d] : 0.0);
+                    }
+    for (int p = 0; p < 24; ++p)
+        for (int t = 0; t < KF; ++t)
+            for (int j = 0; j < NJ; ++j)
+                for (int l = 0; l < 32; ++l) {
+                    const int k = moment_of(NB, t, l % 4), b = 8 * j + l / 4;
+                    tl.push_back(k < NM && b < NB ? T[((size_t)p * NB + b) * NM + k] : 0.0);
+                }
+    std::vector<double> inv_mass(NB), jd(9 * ncell), inv_detj(ncell);
+    for (int j = 0; j < NB; ++j) inv_mass[j] = 1.0 / tab.mass_ref[j];
+    for (int64_t e = 0; e < ncell; ++e) {
+        const double dj = hgeo[10 * e + 9];
+        for (int i = 0; i < 9; ++i) jd[9 * e + i] = dj * hgeo[10 * e + i];
+        inv_detj[e] = 1.0 / dj;
+    }
+    m.nfgroups = (int)fg.size();
+    m.negroups = (int)eg.size();
+    int rc;
+    if ((rc = rows8_upload(m, &m.t.tf, tf)) || (rc = rows8_upload(m, &m.t.tm, tm)) || (rc = rows8_upload(m, &m.t.tv, tv)) ||
+        (rc = rows8_upload(m, &m.t.tw, tw)) || (rc = rows8_upload(m, &m.t.tl, tl)) ||
+        (rc = rows8_upload(m, &m.t.inv_mass, inv_mass)) || (rc = rows8_upload(m, &m.jd, jd)) ||
+        (rc = rows8_upload(m, &m.inv_detj, inv_detj)) || (rc = rows8_upload(m, &m.fgroups, fg)) ||
+        (rc = rows8_upload(m, &m.egroups, eg)))
+        return rc;
+    for (int i = 0; i < 2; ++i) {
+        void* p = nullptr;
+        const size_t n = i ? sizeof(int) : sizeof(double) * nface * 5 * MR;
+        if (cudaMalloc(&p, n) != cudaSuccess) return DG_E_NOMEM;
+        m.bufs.push_back(p);
+        if (cudaMemset(p, 0, n) != cudaSuccess) return DG_E_CUDA;
+        if (i) m.err = (int*)p;
+        else m.rec = (double*)p;
+    }
+    m.ready = true;
+    return DG_OK;
+}
+
+inline void free_rows8(Rows8Data& m) {
+    for (void* p : m.bufs) cudaFree(p);
+    m.bufs.clear();
+    m.ready = false;
+}
+
+}  // namespace fvedg

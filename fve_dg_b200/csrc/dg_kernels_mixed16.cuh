@@ -21,6 +21,7 @@
 #include <cstring>
 
 #include "dg_kernels_mixed.cuh"
+#include "dg_slots.cuh"
 
 namespace fvedg {
 
@@ -105,63 +106,11 @@ struct Mixed16ElemArgs {
 __device__ __forceinline__ uint4 ld_table4(const uint32_t* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
 __device__ __forceinline__ uint2 ld_table2(const uint32_t* p) { return __ldg(reinterpret_cast<const uint2*>(p)); }
 
-// State rows in shared memory, one slot per item. A row that starts on an 8-byte boundary keeps that
-// offset in its slot, so that its middle is one bulk copy (16-byte aligned on both sides) whatever the
-// row length; a first or last double that sticks out is moved by itself. The slot stride spreads the
-// 16-byte accesses of the fragment pattern (eight rows, runs of 80 bytes) over all banks.
+// Slots whose stride spreads the 16-byte accesses of the fragment pattern (eight rows, runs of 80 bytes) over
+// all banks.
+constexpr int slot_unit16(int u) { return u % 8 == 4 ? u : slot_unit16(u + 1); }
 template <int NB>
-struct RowSlots {
-    static constexpr int LEN = 5 * NB;
-    static constexpr int unit(int u) { return u % 8 == 4 ? u : unit(u + 1); }
-    static constexpr int BYTES = 16 * unit((8 * LEN + 8 + 15) / 16);
-    static __device__ __forceinline__ int skew(const double* row) { return (int)(reinterpret_cast<uintptr_t>(row) & 8); }
-    static __device__ __forceinline__ double* at(void* slots, int i, const double* row) {
-        return reinterpret_cast<double*>(static_cast<char*>(slots) + i * BYTES + skew(row));
-    }
-    // Lane `lane` < n: its row into slot `lane`; every such lane announces its own bytes on `bar` (count n).
-    static __device__ __forceinline__ void load(void* slots, int lane, int n, const double* row, uint64_t* bar) {
-        if (lane < n) {
-            double* to = at(slots, lane, row);
-            const int head = skew(row) ? 1 : 0, mid = (LEN - head) & ~1, tail = LEN - head - mid;
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            if (LEN % 2 == 0 && !head) {
-                mbar_arrive_expect_tx(bar, 8u * LEN);
-                bulk_copy_g2s(to, row, 8u * LEN, bar);
-            } else {  // the arrival follows the stores of this lane, which it releases
-                mbar_expect_tx(bar, 8u * mid);
-                bulk_copy_g2s(to + head, row + head, 8u * mid, bar);
-                if (head) to[0] = row[0];
-                if (tail) to[LEN - 1] = row[LEN - 1];
-                mbar_arrive(bar);
-            }
-        }
-    }
-    // Lane `lane` < n: slot `lane` back to its row; the caller has fenced the slots' writes.
-    static __device__ __forceinline__ void store(void* slots, int lane, int n, double* row) {
-        if (lane < n) {
-            double* from = at(slots, lane, row);
-            const int head = skew(row) ? 1 : 0, mid = (LEN - head) & ~1, tail = LEN - head - mid;
-            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(row + head),
-                         "r"(smem_addr(from + head)), "r"(8u * mid)
-                         : "memory");
-            if (head) row[0] = from[0];
-            if (tail) row[LEN - 1] = from[LEN - 1];
-        }
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    }
-};
-
-// Waits for the warp's rows, a bounded number of polls; when they run out, records it, lets the copies in
-// flight land (bounded again) and returns false to the whole warp.
-__device__ __forceinline__ bool rows_landed(uint64_t& bar, unsigned& parity, int* err, int lane) {
-    bool ok = mbar_wait_bounded(&bar, parity, kBulkSpinLimit);
-    if (!ok) {
-        if (lane == 0 && err) atomicExch(err, DG_E_WATCHDOG);
-        mbar_wait_bounded(&bar, parity, kBulkSpinLimit);
-    }
-    parity ^= 1u;
-    return __all_sync(0xffffffffu, ok);
-}
+using RowSlots = RowSlotsOf<NB, 16 * slot_unit16((40 * NB + 8 + 15) / 16)>;
 
 // Ten consecutive doubles (two modes of five variables) of a slot; `two`: the second mode exists.
 __device__ __forceinline__ void slot_pair(double (&d)[10], const double* p, bool vec, bool two) {
