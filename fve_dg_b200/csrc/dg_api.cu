@@ -48,6 +48,13 @@ int upload(T** p, const std::vector<T>& v) {
 }
 }  // namespace
 
+// The viscous operator in rows of eight, orders 1 to 4. Where the context steps Navier-Stokes in FP64: always, the
+// stage is then two fused launches instead of four (a step of 48 cells 84 -> 56 us at P1 and 278 -> 238 at P4, of
+// 4,374 cells 173 -> 68 and 756 -> 277). The operator alone: from one group per SM (1,184 cells), where its two
+// launches are level with those of one warp per item; viscous part of a step at 750 cells, P2: 139 -> 141 us in all,
+// at 1,296: 181 -> 147, at 4,374: 299 -> 175.
+constexpr int kVisc8PerSm = 1;
+
 struct dg_ctx {
     dg_config cfg{};
     int qv = 0, qf = 0;
@@ -78,6 +85,7 @@ struct dg_ctx {
     MixedData mixed;               // mixed-precision form buffers
     TcData tc;                     // FP64 form on the FP64 tensor cores (the configurations' rules)
     Rows8Data rows;                // the same in rows of eight (large meshes, and orders 0 and 5)
+    Visc8Data visc8;               // viscous operator in rows of eight (large meshes)
     bool have_state = false;
     bool has_dirichlet = false;    // some boundary face is Dirichlet: U_D must be set first
     cudaGraphExec_t graph = nullptr;
@@ -365,8 +373,30 @@ int timed(dg_ctx* c, int cls, cudaStream_t s, F&& fn) {
 // The viscous operator's tables (the volume ones transposed so that lanes over points read rows,
 // the A operands of its tensor-core products) and its per-face buffer; made by the first call.
 int viscous_buffers(dg_ctx* c) {
-    if (c->d_visc_vf) return DG_OK;
+    if (c->d_visc_vf || c->visc8.ready) return DG_OK;
     const Tables& t = c->tab;
+    if (c->cfg.order >= 1 && c->cfg.order <= 4 && c->rows.ready) {
+        c->visc8.rows = &c->rows;
+        return init_visc8(c->visc8, t, c->nface, c->qf);
+    }
+    const bool fused = c->cfg.mu > 0.0 && c->cfg.precision == DG_PREC_FP64;
+    if (c->cfg.order >= 1 && c->cfg.order <= 4 && rows8_supported(c->cfg.order, c->qv, c->qf)) {
+        std::vector<FaceInfo> hfi(c->nface);
+        std::vector<ElemFace> hef(4 * c->ncell);
+        std::vector<double> hgeo(10 * c->ncell);
+        std::vector<FaceGroup8> fg;
+        std::vector<ElemGroup8> eg;
+        DG_CUDA(cudaMemcpy(hfi.data(), c->d_fi, sizeof(FaceInfo) * hfi.size(), cudaMemcpyDeviceToHost));
+        DG_CUDA(cudaMemcpy(hef.data(), c->d_ef, sizeof(ElemFace) * hef.size(), cudaMemcpyDeviceToHost));
+        if (rows8_groups(c->cfg.order, c->qv, c->qf, c->sms, hfi, hef, c->nowned, fg, eg, fused ? 0 : kVisc8PerSm)) {
+            DG_CUDA(cudaMemcpy(hgeo.data(), c->d_geo, sizeof(double) * hgeo.size(), cudaMemcpyDeviceToHost));
+            c->visc8.own.sms = c->sms;
+            int rc = init_rows8(c->visc8.own, t, hgeo, fg, eg, c->ncell, c->nface, c->qv, c->qf, false);
+            if (rc) return rc;
+            c->visc8.rows = &c->visc8.own;
+            return init_visc8(c->visc8, t, c->nface, c->qf);
+        }
+    }
     const int nb = t.nb, nqv = t.nqv, nqf = t.nqf;
     std::vector<double> pv((size_t)nb * nqv), dpv((size_t)nb * 3 * nqv);  // volume tables, transposed
     for (int g = 0; g < nqv; ++g)
@@ -401,6 +431,27 @@ int viscous_buffers(dg_ctx* c) {
 }
 
 int viscous_launch(dg_ctx* c, const double* U, double* R, double mu, double prandtl, cudaStream_t s);
+
+// Arguments of the viscous kernels in rows of eight: mode 0 writes the viscous residual, mode 1 (the fused
+// Navier-Stokes kernels) the RK stage.
+Visc8Args visc8_args(dg_ctx* c, const double* U, const double* U0, double* out, int mode, double dt, double a0, double a1,
+                     double mu, double prandtl) {
+    const Rows8Data& r = *c->visc8.rows;
+    Visc8Args v;
+    v.f.U = U; v.f.fi = c->d_fi; v.f.groups = r.fgroups; v.f.ngroups = r.nfgroups; v.f.UD = c->d_UD; v.f.rec = c->visc8.rec;
+    v.f.t = r.t; v.f.gamma = c->cfg.gamma; v.f.flux = c->cfg.flux; v.f.faces_mask = 3; v.f.err = r.err;
+    v.e.U = U; v.e.U0 = U0; v.e.out = out; v.e.rec = c->visc8.rec; v.e.jd = r.jd; v.e.inv_detj = r.inv_detj;
+    v.e.groups = r.egroups; v.e.ngroups = r.negroups; v.e.t = r.t; v.e.gamma = c->cfg.gamma; v.e.with_volume = 1;
+    v.e.mode = mode; v.e.dt = dt; v.e.a0 = a0; v.e.a1 = a1;
+    v.e.dt_inst = mode == 1 ? c->d_dt_inst : nullptr; v.e.elem_inst = c->d_elem_inst; v.e.Rv = nullptr; v.e.err = r.err;
+    v.v = c->visc8.v; v.geo = c->d_geo; v.h = c->d_h; v.mu = mu; v.cq = c->cfg.gamma / prandtl; v.order = c->cfg.order;
+    return v;
+}
+
+// Whether a Navier-Stokes stage runs as the two fused launches (the FP64 form in rows of eight).
+bool fused_navier_stokes(const dg_ctx* c) {
+    return c->cfg.mu > 0.0 && c->cfg.precision == DG_PREC_FP64 && c->visc8.ready;
+}
 
 // Navier-Stokes stepping (dg_config.mu > 0): the viscous residual of the stage input, which the
 // element kernels' update subtracts from the convective one: L = (R_visc - R_conv) / b, as the
@@ -442,7 +493,18 @@ int step_fp64(dg_ctx* c, double dt, cudaStream_t s, int st0, int st1) {
     const double* in[3] = {c->d_Un, c->d_Ua, c->d_Ub};
     double* out[3] = {c->d_Ua, c->d_Ub, c->d_Un};
     for (int st = st0; st < st1; ++st) {
-        int rc = viscous_stage(c, in[st], s);
+        int rc;
+        if (fused_navier_stokes(c)) {
+            const Visc8Args v = visc8_args(c, in[st], c->d_Un, out[st], 1, dt, A0[st], A1[st], c->cfg.mu, c->cfg.prandtl);
+            const Rows8Data& r = *c->visc8.rows;
+            g_launches += 2;
+            if ((rc = timed(c, 0, s, [&] { return visc8_face(r.order, r.qv, r.qf, r.sms, v, true, s); })) ||
+                (rc = timed(c, 1, s, [&] { return visc8_element(r.order, r.qv, r.qf, r.sms, v, true, s); })) ||
+                (rc = limit_stage(c, st, in[st], out[st], s)))
+                return rc;
+            continue;
+        }
+        rc = viscous_stage(c, in[st], s);
         if (rc) return rc;
         rc = timed(c, 0, s, [&] { return fp64_face(c, in[st], 3, s); });
         if (rc) return rc;
@@ -498,7 +560,7 @@ int stage_phase_mixed(dg_ctx* c, double dt, int st, int phase, cudaStream_t s) {
 }
 
 int launches_per_step(const dg_ctx* c) {
-    const int lim = (c->cfg.limiter ? (c->nowned < c->ncell ? 6 : 3) : 0) + (c->cfg.mu > 0.0 ? 6 : 0);
+    const int lim = (c->cfg.limiter ? (c->nowned < c->ncell ? 6 : 3) : 0) + (c->cfg.mu > 0.0 && !fused_navier_stokes(c) ? 6 : 0);
     if (c->cfg.precision == DG_PREC_MIXED) return (c->cfg.schedule == 1 ? 3 : mixed_launches_per_step(c->mixed)) + lim;
     return 6 + lim;
 }
@@ -507,7 +569,7 @@ int launches_per_step(const dg_ctx* c) {
 // waits (DG_OK or DG_E_WATCHDOG); a set word is cleared.
 int check_queue(dg_ctx* c) {
     int err = 0;
-    for (int* word : {c->mixed.err, c->rows.err}) {
+    for (int* word : {c->mixed.err, c->rows.err, c->visc8.own.err}) {
         if (!word) continue;
         if (cudaMemcpy(&err, word, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return DG_E_CUDA;
         if (err != DG_OK) {
@@ -552,6 +614,7 @@ void free_ctx(dg_ctx* c) {
     free_mixed(c->mixed);
     free_tc(c->tc);
     free_rows8(c->rows);
+    free_visc8(c->visc8);
     if (c->d_queue) cudaFree(c->d_queue);
     if (c->d_dt_inst) cudaFree(c->d_dt_inst);
     if (c->d_lim_bnd) cudaFree(c->d_lim_bnd);
@@ -735,7 +798,9 @@ dg_ctx* create_impl(const dg_mesh_desc* mesh, const dg_config* cfg, int* err, co
     }
     // Navier-Stokes stepping: the viscous buffers now, so that no step allocates (graph capture)
     if (cfg->mu > 0.0) {
-        if ((rc = viscous_buffers(c)) || (rc = dev_alloc(&c->d_Rv, (size_t)c->ncell * 5 * nb))) return fail(c, rc);
+        if ((rc = viscous_buffers(c)) ||
+            (rc = dev_alloc(&c->d_Rv, fused_navier_stokes(c) ? 0 : (size_t)c->ncell * 5 * nb)))
+            return fail(c, rc);
         c->mixed.Rv = c->d_Rv;
     }
     // the limiter's per-cell statistics, allocated here so that no step allocates (graph capture)
@@ -945,6 +1010,13 @@ int dg_viscous_residual_device(dg_ctx* c, const double* U, double* R, double mu,
 namespace {
 // The viscous residual of U into R (two launches on stream s); the buffers exist.
 int viscous_launch(dg_ctx* c, const double* U, double* R, double mu, double prandtl, cudaStream_t s) {
+    if (c->visc8.ready) {
+        const Visc8Args v = visc8_args(c, U, U, R, 0, 0.0, 0.0, 0.0, mu, prandtl);
+        const Rows8Data& r = *c->visc8.rows;
+        g_launches += 2;
+        if (const int rc = visc8_face(r.order, r.qv, r.qf, r.sms, v, false, s)) return rc;
+        return visc8_element(r.order, r.qv, r.qf, r.sms, v, false, s);
+    }
     ViscArgs a;
     a.U = U; a.R = R; a.geo = c->d_geo; a.h = c->d_h; a.fi = c->d_fi; a.ef = c->d_ef;
     a.phi_v = c->d_phi_v; a.dphi_v = c->d_dphi_v; a.w_v = c->d_w_v;

@@ -4,6 +4,7 @@
 
 #include "dg_fp64_rows.h"
 #include "dg_mixed_host.cuh"
+#include "dg_viscous_rows.h"
 
 namespace fvedg {
 
@@ -50,16 +51,17 @@ inline int rows8_upload(Rows8Data& m, const T** dst, const std::vector<T>& v) {
 // partial groups).
 inline bool rows8_groups(int order, int qv, int qf, int sms, const std::vector<FaceInfo>& hfi,
                          const std::vector<ElemFace>& hef, int64_t nowned, std::vector<FaceGroup8>& fg,
-                         std::vector<ElemGroup8>& eg) {
+                         std::vector<ElemGroup8>& eg, int per_sm = 5) {
     if (!rows8_supported(order, qv, qf)) return false;
-    if (order >= 1 && order <= 4 && nowned < (int64_t)5 * kRows8 * sms) return false;
+    if (order >= 1 && order <= 4 && nowned < (int64_t)per_sm * kRows8 * sms) return false;
     int inner = 0;
     build_groups(hfi, hef, nowned, fg, eg, &inner);
     return (int64_t)eg.size() * kRows8 * 3 <= nowned * 4 && (int64_t)fg.size() * kRows8 * 3 <= (int64_t)hfi.size() * 4;
 }
 
 inline int init_rows8(Rows8Data& m, const Tables& tab, const std::vector<double>& hgeo, const std::vector<FaceGroup8>& fg,
-                      const std::vector<ElemGroup8>& eg, int64_t ncell, int64_t nface, int qv, int qf) {
+                      const std::vector<ElemGroup8>& eg, int64_t ncell, int64_t nface, int qv, int qf,
+                      bool with_records = true) {
     const int NB = tab.nb, NQV = tab.nqv, NQF = tab.nqf, NM = face_moments(NB), MR = moment_row(NB);
     const int KT = (NB + 3) / 4, NF = pad8(NQF) / 8, NV = pad8(NQV) / 8, NJ = pad8(NB) / 8, MT = (MR + 7) / 8;
     const int KF = moment_ktiles(NB);
@@ -120,7 +122,7 @@ inline int init_rows8(Rows8Data& m, const Tables& tab, const std::vector<double>
         return rc;
     for (int i = 0; i < 2; ++i) {
         void* p = nullptr;
-        const size_t n = i ? sizeof(int) : sizeof(double) * nface * 5 * MR;
+        const size_t n = i ? sizeof(int) : with_records ? sizeof(double) * nface * 5 * MR : 16;
         if (cudaMalloc(&p, n) != cudaSuccess) return DG_E_NOMEM;
         m.bufs.push_back(p);
         if (cudaMemset(p, 0, n) != cudaSuccess) return DG_E_CUDA;
@@ -132,6 +134,76 @@ inline int init_rows8(Rows8Data& m, const Tables& tab, const std::vector<double>
 }
 
 inline void free_rows8(Rows8Data& m) {
+    for (void* p : m.bufs) cudaFree(p);
+    m.bufs.clear();
+    m.ready = false;
+}
+
+// The viscous operator in rows of eight: tables of the derivatives and face records; the tables, groups and
+// status word it shares with the convective kernels are a context's own or built here.
+struct Visc8Data {
+    bool ready = false;
+    Rows8Data own;               // built when the context has no Rows8Data
+    const Rows8Data* rows = nullptr;
+    Visc8Tables v{};
+    double* rec = nullptr;       // [nface][visc_rec(nb)]
+    std::vector<void*> bufs;
+};
+
+inline int init_visc8(Visc8Data& m, const Tables& tab, int64_t nface, int qf) {
+    const int NB = tab.nb, NQV = tab.nqv, NQF = tab.nqf, NM = face_moments(NB);
+    const int KT = (NB + 3) / 4, NF = pad8(NQF) / 8, NV = pad8(NQV) / 8, NJ = pad8(NB) / 8, KD = deriv_ktiles(NB);
+    std::vector<double> psi, norm, tfd, tvd, td;
+    face_moment_basis(tab.order, qf, psi, norm);
+    const double* r = tri_rule(qf);
+    for (int p = 0; p < 24; ++p)
+        for (int nt = 0; nt < NF; ++nt)
+            for (int kt = 0; kt < KT; ++kt)
+                for (int d = 0; d < 3; ++d)
+                    for (int l = 0; l < 32; ++l) {
+                        const int g = 8 * nt + l / 4, b = 4 * kt + l % 4;
+                        tfd.push_back(g < NQF && b < NB ? tab.dphi_f[(((size_t)p * NQF + g) * NB + b) * 3 + d] : 0.0);
+                    }
+    for (int nt = 0; nt < NV; ++nt)
+        for (int kt = 0; kt < KT; ++kt)
+            for (int d = 0; d < 3; ++d)
+                for (int l = 0; l < 32; ++l) {
+                    const int g = 8 * nt + l / 4, b = 4 * kt + l % 4;
+                    tvd.push_back(g < NQV && b < NB ? tab.dphi_v[((size_t)g * NB + b) * 3 + d] : 0.0);
+                }
+    // D[perm][d][j][m] = sum_g w_g dphi_j,d psi_m / |psi_m|^2; degree P - 1, so moments past that vanish
+    const int nd = tab.order * (tab.order + 1) / 2;
+    for (int p = 0; p < 24; ++p)
+        for (int d = 0; d < 3; ++d)
+            for (int t = 0; t < KD; ++t)
+                for (int j = 0; j < NJ; ++j)
+                    for (int l = 0; l < 32; ++l) {
+                        const int k = 8 * (t / 2) + 2 * (l % 4) + t % 2, b = 8 * j + l / 4;
+                        long double s = 0;
+                        if (k < std::min(nd, NM) && b < NB)
+                            for (int g = 0; g < NQF; ++g)
+                                s += (long double)r[3 * g + 2] * tab.dphi_f[(((size_t)p * NQF + g) * NB + b) * 3 + d] * psi[(size_t)k * NQF + g];
+                        td.push_back(k < std::min(nd, NM) && b < NB ? (double)(s / norm[k]) : 0.0);
+                    }
+    auto up = [&](const double** dst, const std::vector<double>& v) {
+        void* p = nullptr;
+        if (cudaMalloc(&p, sizeof(double) * v.size()) != cudaSuccess) return (int)DG_E_NOMEM;
+        m.bufs.push_back(p);
+        *dst = (const double*)p;
+        return cudaMemcpy(p, v.data(), sizeof(double) * v.size(), cudaMemcpyHostToDevice) == cudaSuccess ? (int)DG_OK : (int)DG_E_CUDA;
+    };
+    int rc;
+    if ((rc = up(&m.v.tfd, tfd)) || (rc = up(&m.v.tvd, tvd)) || (rc = up(&m.v.td, td))) return rc;
+    void* p = nullptr;
+    if (cudaMalloc(&p, sizeof(double) * nface * visc_rec(NB)) != cudaSuccess) return DG_E_NOMEM;
+    m.bufs.push_back(p);
+    m.rec = (double*)p;
+    m.ready = true;
+    return DG_OK;
+}
+
+inline void free_visc8(Visc8Data& m) {
+    free_rows8(m.own);
     for (void* p : m.bufs) cudaFree(p);
     m.bufs.clear();
     m.ready = false;
