@@ -752,7 +752,7 @@ dg_ctx* create_impl(const dg_mesh_desc* mesh, const dg_config* cfg, int* err, co
     std::vector<FaceGroup8> fg8;
     std::vector<ElemGroup8> eg8;
     const bool rows = cfg->precision == DG_PREC_FP64 &&
-                      rows8_groups(cfg->order, qv, qf, c->sms, hfi, hef, c->nowned, fg8, eg8);
+                      rows8_groups(cfg->order, qv, qf, c->sms, hfi, hef, c->nowned, fg8, eg8, rows8_per_sm(cfg->order));
     if ((rc = upload(&c->d_h, hh)) || (rc = upload(&c->d_dphi_v, c->tab.dphi_v)) ||
         (rc = upload(&c->d_dphi_f, c->tab.dphi_f)))
         return fail(c, rc);

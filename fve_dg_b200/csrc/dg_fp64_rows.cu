@@ -30,8 +30,7 @@ int run_face(int sms, const Rows8FaceArgs& a, cudaStream_t s) {
     constexpr size_t smem = sizeof(FaceSmem8<NB>) * W;
     static unsigned long long done = 0;
     if (const int rc = opt_in(face_flux_rows8<NB, NQF, W>, smem, done)) return rc;
-    if (a.ngroups > 0) face_flux_rows8<NB, NQF, W><<<std::min(a.ngroups, sms), W * 32, smem, s>>>(a);
-    return cuda_status(cudaGetLastError());
+    return a.ngroups > 0 ? launch_early(face_flux_rows8<NB, NQF, W>, std::min(a.ngroups, sms), W * 32, smem, s, a) : (int)DG_OK;
 }
 
 template <int NB, int NQV>
@@ -40,8 +39,7 @@ int run_element(int sms, const Rows8ElemArgs& a, cudaStream_t s) {
     constexpr size_t smem = sizeof(ElemSmem8<NB>) * W;
     static unsigned long long done = 0;
     if (const int rc = opt_in(element_rows8<NB, NQV, W>, smem, done)) return rc;
-    if (a.ngroups > 0) element_rows8<NB, NQV, W><<<std::min(a.ngroups, sms), W * 32, smem, s>>>(a);
-    return cuda_status(cudaGetLastError());
+    return a.ngroups > 0 ? launch_early(element_rows8<NB, NQV, W>, std::min(a.ngroups, sms), W * 32, smem, s, a) : (int)DG_OK;
 }
 
 }  // namespace

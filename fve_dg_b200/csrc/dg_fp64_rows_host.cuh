@@ -45,15 +45,17 @@ inline int rows8_upload(Rows8Data& m, const T** dst, const std::vector<T>& v) {
 // Whether a mesh runs in rows of eight, with its groups. Orders 0 and 5 have no other tensor-core kernels and
 // always do (P0 56 -> 39 us a step at n = 4 against the runtime-size kernels, P5 326 -> 233; n = 24: 372 -> 260 and
 // 16,345 -> 4,838). For the others groups of three are the faster on small meshes, where a warp's chain of work
-// decides (us a step, three / eight: P1 29 / 34 at n = 4, 31 / 34 at n = 8, 44 / 44 at n = 11, 76 / 71 at n = 14; P2
-// 43 / 46, 62 / 65, 109 / 108 from n = 8; P3 78 / 75, 125 / 118, 231 / 206; P4 115 / 122, 252 / 192, 451 / 372): five
-// groups per SM, about 6,000 cells. And the groups must be reasonably full (many classes of face maps leave as many
-// partial groups).
+// decides (us a step, three / eight: P1 31 / 36 at n = 8, 34 / 36 at n = 9, 42 / 40 at n = 11; P2 54 / 54 at n = 6,
+// 60 / 56 at n = 8, 64 / 58 at n = 9; P3 68 / 74, 80 / 79, 93 / 81; P4 103 / 127, 131 / 134, 177 / 140): five groups per
+// SM at P1, about 6,000 cells, three above. And the groups must be reasonably full (many classes of face maps leave
+// as many partial groups).
+inline int rows8_per_sm(int order) { return order == 0 || order == 5 ? 0 : order == 1 ? 5 : 3; }
+
 inline bool rows8_groups(int order, int qv, int qf, int sms, const std::vector<FaceInfo>& hfi,
                          const std::vector<ElemFace>& hef, int64_t nowned, std::vector<FaceGroup8>& fg,
-                         std::vector<ElemGroup8>& eg, int per_sm = 5) {
+                         std::vector<ElemGroup8>& eg, int per_sm) {
     if (!rows8_supported(order, qv, qf)) return false;
-    if (order >= 1 && order <= 4 && nowned < (int64_t)per_sm * kRows8 * sms) return false;
+    if (nowned < (int64_t)per_sm * kRows8 * sms) return false;
     int inner = 0;
     build_groups(hfi, hef, nowned, fg, eg, &inner);
     return (int64_t)eg.size() * kRows8 * 3 <= nowned * 4 && (int64_t)fg.size() * kRows8 * 3 <= (int64_t)hfi.size() * 4;

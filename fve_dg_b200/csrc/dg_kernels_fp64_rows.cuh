@@ -18,6 +18,7 @@
 #include "dg_flux.cuh"
 #include "dg_kernels_fp64.cuh"
 #include "dg_kernels_mixed16.cuh"
+#include "dg_launch.cuh"
 #include "dg_slots.cuh"
 
 namespace fvedg {
@@ -214,8 +215,10 @@ __global__ void __launch_bounds__(WARPS * 32, 1) face_flux_rows8(Rows8FaceArgs a
     if (lane == 0) mbar_init(&bars[warp], 16);
     __syncwarp();
     unsigned parity = 0;
-    for (int gi = blockIdx.x + gridDim.x * warp; gi < a.ngroups; gi += gridDim.x * WARPS)
+    for (int gi = blockIdx.x + gridDim.x * warp + await_previous(); gi < a.ngroups; gi += gridDim.x * WARPS) {
+        if (gi + gridDim.x * WARPS >= a.ngroups) release_next();
         if (!face_group8<NB, NQF>(a, gi, sm, bars[warp], parity, lane)) break;
+    }
 }
 
 // ---- elements --------------------------------------------------------------------------------------
@@ -365,7 +368,7 @@ __device__ __forceinline__ bool element_group8(const Rows8ElemArgs& a, int gi, E
                 #pragma unroll
                 for (int k = 0; k < 5; ++k) {
                     double R = acc[k][j][i];
-                    if (a.Rv) R -= __ldg(a.Rv + e * B5 + 5 * b + k);
+                    if (a.Rv) R -= a.Rv[e * B5 + 5 * b + k];
                     const double x = row[5 * b + k] - s * R;
                     os[5 * b + k] = u0 ? fma(a.a1, x, a.a0 * row0[5 * b + k]) : a.a1 * x;
                 }
@@ -391,8 +394,10 @@ __global__ void __launch_bounds__(WARPS * 32, 1) element_rows8(Rows8ElemArgs a) 
     if (lane == 0) mbar_init(&bars[warp], 16);
     __syncwarp();
     unsigned parity = 0;
-    for (int gi = blockIdx.x + gridDim.x * warp; gi < a.ngroups; gi += gridDim.x * WARPS)
+    for (int gi = blockIdx.x + gridDim.x * warp + await_previous(); gi < a.ngroups; gi += gridDim.x * WARPS) {
+        if (gi + gridDim.x * WARPS >= a.ngroups) release_next();
         if (!element_group8<NB, NQV>(a, gi, sm, bars[warp], parity, lane)) break;
+    }
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 

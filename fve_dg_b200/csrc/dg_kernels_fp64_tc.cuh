@@ -26,9 +26,20 @@
 
 #include "dg_flux.cuh"
 #include "dg_kernels_fp64.cuh"
+#include "dg_launch.cuh"
 #include "dg_mixed_host.cuh"
 
 namespace fvedg {
+
+// Up to P1 the kernels are launched early (dg_launch.cuh; a step of 3,072 cells 35.0 -> 31.1 us). From P2 on what
+// that saves is lost on their loads, which then can't take the read-only path (P2 at 384 cells 49.5 -> 51.7 us, P4 94.6
+// -> 101).
+__host__ __device__ constexpr bool early_tc(int nb) { return nb <= 4; }
+template <bool EARLY>
+__device__ __forceinline__ double ld_input(const double* p) {
+    if constexpr (EARLY) return ld_earlier(p);
+    else return __ldg(p);
+}
 
 __host__ __device__ constexpr int pad4(int x) { return (x + 3) / 4 * 4; }
 // A shared-memory row stride >= n with stride % 16 == 8 doubles: the 16-byte stores of the
@@ -177,7 +188,7 @@ __device__ __forceinline__ void face_group_tc(const TcFaceArgs& a, int gi, TcFac
             #pragma unroll
             for (int kt = 0; kt < KT; ++kt) {
                 const int b = 4 * kt + tq;
-                A[mt][kt] = (row && b < NB) ? __ldg(a.U + TCK(row - a.U + 5 * b, a.chk.nU, 6)) : 0.0;
+                A[mt][kt] = (row && b < NB) ? ld_input<early_tc(NB)>(a.U + TCK(row - a.U + 5 * b, a.chk.nU, 6)) : 0.0;
             }
         }
         const double* tb = a.t.tf + (int64_t)(s ? perm1 : perm0) * GP * BP;
@@ -232,8 +243,9 @@ template <int NB, int NQF, int W>
 __global__ void TC_FACE_BOUNDS(W, NB) face_flux_tc(TcFaceArgs a) {
     __shared__ TcFaceSmem<NB, NQF> sm[W];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int gi = blockIdx.x * W + warp; gi < a.ngroups; gi += gridDim.x * W)
+    for (int gi = blockIdx.x * W + warp + (early_tc(NB) ? await_previous() : 0); gi < a.ngroups; gi += gridDim.x * W)
         face_group_tc<NB, NQF>(a, gi, sm[warp], lane);
+    if (early_tc(NB)) release_next();
 }
 
 // ---- elements ----------------------------------------------------------------------------------
@@ -283,7 +295,7 @@ __device__ __forceinline__ void element_group_tc(const TcElemArgs& a, int gi, Tc
                 #pragma unroll
                 for (int kt = 0; kt < KT; ++kt) {
                     const int b = 4 * kt + tq;
-                    A[mt][kt] = (row && b < NB) ? __ldg(a.U + TCK(row - a.U + 5 * b, a.chk.nU, 12)) : 0.0;
+                    A[mt][kt] = (row && b < NB) ? ld_input<early_tc(NB)>(a.U + TCK(row - a.U + 5 * b, a.chk.nU, 12)) : 0.0;
                 }
             }
             #pragma unroll
@@ -372,8 +384,8 @@ __device__ __forceinline__ void element_group_tc(const TcElemArgs& a, int gi, Tc
         const double* tl = a.t.tl + (int64_t)(meta & 0xff) * JP * GP;
         #pragma unroll
         for (int kt = 0; kt < GP / 4; ++kt) {
-            const double a0 = rowp[0][q] ? sgn * __ldg(a.Fh + TCK(rowp[0][q] - a.Fh + 4 * kt + tq, a.chk.nFh, 16)) : 0.0;
-            const double a1 = rowp[1][q] ? sgn * __ldg(a.Fh + TCK(rowp[1][q] - a.Fh + 4 * kt + tq, a.chk.nFh, 17)) : 0.0;
+            const double a0 = rowp[0][q] ? sgn * ld_input<early_tc(NB)>(a.Fh + TCK(rowp[0][q] - a.Fh + 4 * kt + tq, a.chk.nFh, 16)) : 0.0;
+            const double a1 = rowp[1][q] ? sgn * ld_input<early_tc(NB)>(a.Fh + TCK(rowp[1][q] - a.Fh + 4 * kt + tq, a.chk.nFh, 17)) : 0.0;
             #pragma unroll
             for (int nt = 0; nt < NJ; ++nt) {
                 const double b = __ldg(a.t.tl + TCK(tl - a.t.tl + (8 * nt + gid) * GP + 4 * kt + tq, a.chk.ntl, 18));
@@ -399,9 +411,9 @@ __device__ __forceinline__ void element_group_tc(const TcElemArgs& a, int gi, Tc
         if (a.mode == 0) {
             a.out[idx] = R;
         } else {
-            if (a.Rv) R -= __ldg(a.Rv + idx);
-            const double u0 = a.a0 != 0.0 ? a.a0 * __ldg(a.U0 + idx) : 0.0;
-            a.out[idx] = u0 + a.a1 * (__ldg(a.U + idx) - sm.sDT[el] * s_inv_mass[j] * R);
+            if (a.Rv) R -= ld_input<early_tc(NB)>(a.Rv + idx);
+            const double u0 = a.a0 != 0.0 ? a.a0 * ld_input<early_tc(NB)>(a.U0 + idx) : 0.0;
+            a.out[idx] = u0 + a.a1 * (ld_input<early_tc(NB)>(a.U + idx) - sm.sDT[el] * s_inv_mass[j] * R);
         }
     }
     __syncwarp();
@@ -415,8 +427,9 @@ __global__ void TC_ELEM_BOUNDS(W, NB) element_tc(TcElemArgs a) {
     __syncthreads();
     auto& sm = reinterpret_cast<TcElemSmem<NB, NQV>*>(smem_raw)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    for (int gi = blockIdx.x * W + (threadIdx.x >> 5); gi < a.ngroups; gi += gridDim.x * W)
+    for (int gi = blockIdx.x * W + (threadIdx.x >> 5) + (early_tc(NB) ? await_previous() : 0); gi < a.ngroups; gi += gridDim.x * W)
         element_group_tc<NB, NQV, NQF>(a, gi, sm, s_inv_mass, lane);
+    if (early_tc(NB)) release_next();
 }
 
 // ---- host side ---------------------------------------------------------------------------------
@@ -546,16 +559,15 @@ inline int tc_launch(TcData& m, int which, const TcFaceArgs& fa, const TcElemArg
     constexpr int W = 4;
     if (which == 0) {
         const int g = (int)std::min<int64_t>((fa.ngroups + W - 1) / W, (int64_t)m.sms * 32);
-        if (g > 0) face_flux_tc<NB, NQF, W><<<g, W * 32, 0, s>>>(fa);
+        return g > 0 ? launch_as<early_tc(NB)>(face_flux_tc<NB, NQF, W>, g, W * 32, 0, s, fa) : (int)DG_OK;
     } else {
         constexpr size_t smem = sizeof(TcElemSmem<NB, NQV>) * W;
         static unsigned long long done = 0;
         int rc = ensure_smem(element_tc<NB, NQV, NQF, W>, smem, done);
         if (rc) return rc;
         const int g = (int)std::min<int64_t>((ea.ngroups + W - 1) / W, (int64_t)m.sms * 32);
-        if (g > 0) element_tc<NB, NQV, NQF, W><<<g, W * 32, smem, s>>>(ea);
+        return g > 0 ? launch_as<early_tc(NB)>(element_tc<NB, NQV, NQF, W>, g, W * 32, smem, s, ea) : (int)DG_OK;
     }
-    return cuda_status(cudaGetLastError());
 }
 
 inline int tc_kernel(TcData& m, int which, const TcFaceArgs& fa, const TcElemArgs& ea, cudaStream_t s) {

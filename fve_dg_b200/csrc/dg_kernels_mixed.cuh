@@ -44,6 +44,7 @@
 #include "dg_flux.cuh"
 #include "dg_internal.h"
 #include "dg_kernels_fp64.cuh"
+#include "dg_launch.cuh"
 #include "dg_tma.cuh"
 
 namespace fvedg {
@@ -192,29 +193,25 @@ struct AFrag {
     uint32_t th[2], tl[2];
 };
 
-// Rows gid and gid + 8 from A rows in global memory (null: a zero row). `Coherent` reads through
-// L2 only, for data written earlier in the same launch (the persistent schedule).
-template <int K, bool Coherent>
+// Rows gid and gid + 8 from A rows in global memory (null: a zero row), through L2 only: they may have been written
+// earlier in the same launch (the persistent schedule).
+template <int K>
 __device__ __forceinline__ void load_afrag(AFrag<K>& A, const uint32_t* r0, const uint32_t* r1, int lane,
                                            uint32_t flip = 0u) {
     const int tq = lane & 3;
     #pragma unroll
     for (int t = 0; t < KTiles<K>::N16; ++t) {
         uint4 v0 = make_uint4(0u, 0u, 0u, 0u), v1 = v0;
-        if (r0) v0 = Coherent ? __ldcg(reinterpret_cast<const uint4*>(r0 + t * 16 + tq * 4))
-                              : __ldg(reinterpret_cast<const uint4*>(r0 + t * 16 + tq * 4));
-        if (r1) v1 = Coherent ? __ldcg(reinterpret_cast<const uint4*>(r1 + t * 16 + tq * 4))
-                              : __ldg(reinterpret_cast<const uint4*>(r1 + t * 16 + tq * 4));
+        if (r0) v0 = __ldcg(reinterpret_cast<const uint4*>(r0 + t * 16 + tq * 4));
+        if (r1) v1 = __ldcg(reinterpret_cast<const uint4*>(r1 + t * 16 + tq * 4));
         A.h[t][0] = v0.x ^ flip; A.h[t][1] = v1.x ^ flip; A.h[t][2] = v0.y ^ flip; A.h[t][3] = v1.y ^ flip;
         A.l[t][0] = v0.z ^ flip; A.l[t][1] = v1.z ^ flip; A.l[t][2] = v0.w ^ flip; A.l[t][3] = v1.w ^ flip;
     }
     if constexpr (KTiles<K>::TAIL) {
         constexpr int o = KTiles<K>::N16 * 16;
         uint2 u0 = make_uint2(0u, 0u), u1 = u0;
-        if (r0) u0 = Coherent ? __ldcg(reinterpret_cast<const uint2*>(r0 + o + tq * 2))
-                              : __ldg(reinterpret_cast<const uint2*>(r0 + o + tq * 2));
-        if (r1) u1 = Coherent ? __ldcg(reinterpret_cast<const uint2*>(r1 + o + tq * 2))
-                              : __ldg(reinterpret_cast<const uint2*>(r1 + o + tq * 2));
+        if (r0) u0 = __ldcg(reinterpret_cast<const uint2*>(r0 + o + tq * 2));
+        if (r1) u1 = __ldcg(reinterpret_cast<const uint2*>(r1 + o + tq * 2));
         A.th[0] = u0.x ^ flip; A.th[1] = u1.x ^ flip;
         A.tl[0] = u0.y ^ flip; A.tl[1] = u1.y ^ flip;
     }
@@ -229,7 +226,7 @@ __device__ __forceinline__ void load_afrag_state(AFrag<K>& A, const double* r0, 
     auto v = [&](const double* r, int x) -> float {
         if (!r || x + 1 >= NB) return 0.f;
         if constexpr (SMEM) return (float)r[5 * (x + 1)];
-        else return (float)__ldg(r + 5 * (x + 1));
+        else return (float)r[5 * (x + 1)];
     };
     #pragma unroll
     for (int t = 0; t < KTiles<K>::N16; ++t) {
@@ -313,7 +310,7 @@ __device__ __forceinline__ void face_group_mixed(const MixedFaceArgs& a, int gi,
         float v = 0.f;
         if (r < 5 * grp.n) {
             const FaceInfo& F = a.fi[grp.f[r / 5]];
-            v = (float)__ldg(a.U + (int64_t)(s ? F.c1 : F.c0) * (5 * NB) + r % 5);
+            v = (float)a.U[(int64_t)(s ? F.c1 : F.c0) * (5 * NB) + r % 5];
         }
         sm.sC0[s][r] = v;
     }
@@ -321,7 +318,7 @@ __device__ __forceinline__ void face_group_mixed(const MixedFaceArgs& a, int gi,
         const FaceInfo& F = a.fi[grp.f[lane]];
         float c0[5], n[3], Fn[5], rho, vel[3], p;
         #pragma unroll
-        for (int k = 0; k < 5; ++k) c0[k] = (float)__ldg(a.U + (int64_t)F.c0 * (5 * NB) + k);
+        for (int k = 0; k < 5; ++k) c0[k] = (float)a.U[(int64_t)F.c0 * (5 * NB) + k];
         #pragma unroll
         for (int i = 0; i < 3; ++i) n[i] = (float)F.n[i];
         const float jw = (float)F.jw;
@@ -417,8 +414,9 @@ template <int NB, int NQF, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, NB <= 20 ? 36 / WARPS : 24 / WARPS) face_flux_mixed(MixedFaceArgs a) {
     __shared__ FaceMixedSmem<NQF> sm[WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int gi = blockIdx.x * WARPS + warp; gi < a.ngroups; gi += gridDim.x * WARPS)
+    for (int gi = blockIdx.x * WARPS + warp + await_previous(); gi < a.ngroups; gi += gridDim.x * WARPS)
         face_group_mixed<NB, NQF>(a, gi, sm[warp], lane);
+    release_next();
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -518,7 +516,7 @@ __device__ __forceinline__ void element_group_mixed(const MixedElemArgs& a, int 
                 reinterpret_cast<const char*>(a.U + (int64_t)grp.e[el] * 5 * NB) + part * 128));
         }
     }
-    if (lane < 16) sm.sC0[lane] = lane < 5 * ne ? (float)__ldg(a.U + (int64_t)grp.e[lane / 5] * (5 * NB) + lane % 5) : 0.f;
+    if (lane < 16) sm.sC0[lane] = lane < 5 * ne ? (float)a.U[(int64_t)grp.e[lane / 5] * (5 * NB) + lane % 5] : 0.f;
     if (lane < ne) {
         const int e = grp.e[lane];
         sm.sE[lane] = e;
@@ -531,7 +529,7 @@ __device__ __forceinline__ void element_group_mixed(const MixedElemArgs& a, int 
         const double* geo = a.geo + e * 10;
         double c[5], J[9];
         #pragma unroll
-        for (int i = 0; i < 5; ++i) c[i] = __ldg(a.U + e * (5 * NB) + i);
+        for (int i = 0; i < 5; ++i) c[i] = a.U[e * (5 * NB) + i];
         #pragma unroll
         for (int i = 0; i < 9; ++i) J[i] = __ldg(geo + i);
         const double dj = __ldg(geo + 9);
@@ -640,7 +638,7 @@ __device__ __forceinline__ void element_group_mixed(const MixedElemArgs& a, int 
     // face integrals: the flux deviations arrive split, in fragment order; side 1 negated exactly
     auto face_rows = [&](AFrag<KF>& A, int q) {
         const uint32_t flip = (grp.meta[q] >> 8) ? 0x80008000u : 0u;
-        load_afrag<KF, true>(A, v0 ? a.dev + (int64_t)grp.face[r0 / 5][q] * FR + (r0 % 5) * KF : nullptr,
+        load_afrag<KF>(A, v0 ? a.dev + (int64_t)grp.face[r0 / 5][q] * FR + (r0 % 5) * KF : nullptr,
                              v1 ? a.dev + (int64_t)grp.face[r1 / 5][q] * FR + (r1 % 5) * KF : nullptr, lane, flip);
     };
     #pragma unroll
@@ -718,7 +716,7 @@ __device__ __forceinline__ void element_group_mixed(const MixedElemArgs& a, int 
                 const int i = lane + 32 * (b0 + j);
                 const int el = i / (5 * NB), r = i - el * (5 * NB);
                 ix[j] = i < ndof ? (int64_t)sm.sE[el] * (5 * NB) + r : -1;
-                uu[j] = ix[j] >= 0 ? __ldg(a.U + ix[j]) : 0.0;
+                uu[j] = ix[j] >= 0 ? a.U[ix[j]] : 0.0;
                 vv[j] = (ix[j] >= 0 && u0) ? a.U0[ix[j]] : 0.0;
             }
             #pragma unroll
@@ -1011,10 +1009,11 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) element_mixed_staged(MixedEl
     element_tables_init(tabs, a.t.inv_mass);  // ends in __syncthreads: the barriers are initialised
     const ElemBTabs bt{a.t.tva, a.t.tvp, a.t.tfl};
     unsigned parity = 0;
-    for (int gi = blockIdx.x * WARPS + warp; gi < a.ngroups; gi += gridDim.x * WARPS) {
+    for (int gi = blockIdx.x * WARPS + warp + await_previous(); gi < a.ngroups; gi += gridDim.x * WARPS) {
         if (!element_group_staged<NB, NQV, NQF>(a, gi, sm, st, tabs, lane, bt, parity)) break;
         parity ^= 1u;
     }
+    release_next();
 }
 
 template <int NB, int NQV, int NQF>
@@ -1043,8 +1042,9 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 3 : 6) element_mixed(
     S& sm = reinterpret_cast<S*>(smem_raw)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const ElemBTabs bt{a.t.tva, a.t.tvp, a.t.tfl};
-    for (int gi = blockIdx.x * WARPS + (threadIdx.x >> 5); gi < a.ngroups; gi += gridDim.x * WARPS)
+    for (int gi = blockIdx.x * WARPS + (threadIdx.x >> 5) + await_previous(); gi < a.ngroups; gi += gridDim.x * WARPS)
         element_group_mixed<NB, NQV, NQF>(a, gi, sm, tabs, lane, bt);
+    release_next();
 }
 
 }  // namespace fvedg

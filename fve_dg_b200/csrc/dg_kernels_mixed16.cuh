@@ -459,8 +459,9 @@ __global__ void __launch_bounds__(WARPS * 32, 1) face_flux_mixed16(Mixed16FaceAr
     if (lane == 0) mbar_init(&bars[warp], kRows);
     __syncwarp();
     unsigned parity = 0;
-    face_run16<NB, NQF>(a, blockIdx.x * WARPS + warp, a.ngroups, gridDim.x * WARPS,
+    face_run16<NB, NQF>(a, blockIdx.x * WARPS + warp + await_previous(), a.ngroups, gridDim.x * WARPS,
                         reinterpret_cast<FaceSmem16<NB, NQF>*>(smem_raw)[warp], bars[warp], parity, lane);
+    if (NB <= 20) release_next();  // at P4 the next kernel's blocks took L1 from the last items (440 -> 467 us a step)
 }
 
 // ---- elements --------------------------------------------------------------------------------------
@@ -738,7 +739,7 @@ __device__ __forceinline__ bool element_group16(const Mixed16ElemArgs& a, const 
             const uint32_t* r0 = a.rec + (int64_t)grp.face[gid][q] * RW;
             const uint32_t* r1 = a.rec + (int64_t)grp.face[gid + 8][q] * RW;
             #pragma unroll
-            for (int k = 0; k < 5; ++k) load_afrag<KM, true>(F[k], r0 + k * KM, r1 + k * KM, lane, flip);
+            for (int k = 0; k < 5; ++k) load_afrag<KM>(F[k], r0 + k * KM, r1 + k * KM, lane, flip);
             const uint32_t* tb = t.tfl + (grp.meta[q] & 0xff) * NJ * KTiles<KM>::NT_U32;
             #pragma unroll
             for (int j = 0; j < NJ; ++j) {
@@ -901,9 +902,10 @@ __global__ void __launch_bounds__(WARPS * 32, 1) element_mixed16(Mixed16ElemArgs
     if (lane == 0) mbar_init(&bars[warp], kRows);
     __syncthreads();
     unsigned parity = 0;
-    elem_run16<NB, NQV>(a, t, blockIdx.x * WARPS + warp, a.ngroups, gridDim.x * WARPS,
+    elem_run16<NB, NQV>(a, t, blockIdx.x * WARPS + warp + await_previous(), a.ngroups, gridDim.x * WARPS,
                         reinterpret_cast<ElemSmem16<NB, NQV>*>(smem_raw + ElemSizes16<NB, NQV>::tables)[warp],
                         bars[warp], parity, lane);
+    if (NB <= 20) release_next();
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 

@@ -74,8 +74,7 @@ int run_face(int sms, const Mixed16FaceArgs& a, cudaStream_t s) {
     constexpr size_t smem = sizeof(FaceSmem16<NB, NQF>) * W;
     static unsigned long long done = 0;
     if (const int rc = opt_in(face_flux_mixed16<NB, NQF, W>, smem, done)) return rc;
-    if (a.ngroups > 0) face_flux_mixed16<NB, NQF, W><<<std::min((a.ngroups + W - 1) / W, sms), W * 32, smem, s>>>(a);
-    return cuda_status(cudaGetLastError());
+    return a.ngroups > 0 ? launch_early(face_flux_mixed16<NB, NQF, W>, std::min((a.ngroups + W - 1) / W, sms), W * 32, smem, s, a) : (int)DG_OK;
 }
 
 template <int NB, int NQV>
@@ -84,8 +83,7 @@ int run_element(int sms, const Mixed16ElemArgs& a, cudaStream_t s) {
     constexpr size_t smem = ElemSizes16<NB, NQV>::tables + sizeof(ElemSmem16<NB, NQV>) * W;
     static unsigned long long done = 0;
     if (const int rc = opt_in(element_mixed16<NB, NQV, W>, smem, done)) return rc;
-    if (a.ngroups > 0) element_mixed16<NB, NQV, W><<<std::min((a.ngroups + W - 1) / W, sms), W * 32, smem, s>>>(a);
-    return cuda_status(cudaGetLastError());
+    return a.ngroups > 0 ? launch_early(element_mixed16<NB, NQV, W>, std::min((a.ngroups + W - 1) / W, sms), W * 32, smem, s, a) : (int)DG_OK;
 }
 
 template <int NB, int NQV, int NQF>

@@ -459,7 +459,7 @@ inline int mixed_launch(MixedData& m, int which, const double* U, const double* 
         constexpr int W = 4;  // 4-warp CTAs: finer-grained scheduling than 8 at the same occupancy
         const int n = g1 < 0 ? m.nfgroups : g1 - g0;
         const int g = (int)std::min<int64_t>((n + W - 1) / W, (int64_t)m.sms * 64);
-        face_flux_mixed<NB, NQF, W><<<g, W * 32, 0, s>>>(face_args(m, U, face_mask, g0, g1));
+        return launch_early(face_flux_mixed<NB, NQF, W>, g, W * 32, 0, s, face_args(m, U, face_mask, g0, g1));
     } else if (m.elem_kernel == 2 && (5 * NB * 8) % 16 == 0 && ((uintptr_t)U & 15) == 0 &&
                ((uintptr_t)U0 & 15) == 0) {
         if constexpr ((5 * NB * 8) % 16 == 0) {
@@ -471,7 +471,7 @@ inline int mixed_launch(MixedData& m, int which, const double* U, const double* 
                 int rc = ensure_smem(element_mixed_staged<NB, NQV, NQF, W, 2>, smem, done);
                 if (rc) return rc;
                 const int g = (int)std::min<int64_t>((m.negroups + W - 1) / W, (int64_t)m.sms * 2);
-                element_mixed_staged<NB, NQV, NQF, W, 2><<<g, W * 32, smem, s>>>(ea);
+                return launch_early(element_mixed_staged<NB, NQV, NQF, W, 2>, g, W * 32, smem, s, ea);
             } else {
                 constexpr int W = elem_staged_warps<NB, NQV, NQF>(1);
                 constexpr size_t smem = elem_staged_warp_smem<NB, NQV, NQF>() * W;
@@ -479,7 +479,7 @@ inline int mixed_launch(MixedData& m, int which, const double* U, const double* 
                 int rc = ensure_smem(element_mixed_staged<NB, NQV, NQF, W, 1>, smem, done);
                 if (rc) return rc;
                 const int g = (int)std::min<int64_t>((m.negroups + W - 1) / W, (int64_t)m.sms);
-                element_mixed_staged<NB, NQV, NQF, W, 1><<<g, W * 32, smem, s>>>(ea);
+                return launch_early(element_mixed_staged<NB, NQV, NQF, W, 1>, g, W * 32, smem, s, ea);
             }
         }
     } else {
@@ -488,10 +488,10 @@ inline int mixed_launch(MixedData& m, int which, const double* U, const double* 
         int rc = ensure_smem(element_mixed<NB, NQV, NQF, WE>, smem, done);
         if (rc) return rc;
         const int g = (int)std::min<int64_t>((m.negroups + WE - 1) / WE, (int64_t)m.sms * 32);
-        element_mixed<NB, NQV, NQF, WE><<<g, WE * 32, smem, s>>>(
-            elem_args(m, U, U0, out, mode, dt, a0, a1, with_volume));
+        return launch_early(element_mixed<NB, NQV, NQF, WE>, g, WE * 32, smem, s,
+                            elem_args(m, U, U0, out, mode, dt, a0, a1, with_volume));
     }
-    return cuda_status(cudaGetLastError());
+    return DG_E_ARG;  // staged, of a row length that excludes it: not reached
 }
 
 // Element-kernel shapes of the two-launch schedule that dg_autotune times: the kernel (0: loads

@@ -26,8 +26,7 @@ int run_face(int sms, const Visc8Args& a, cudaStream_t s) {
     constexpr size_t smem = sizeof(FaceSmem8<NB>) * W;
     static unsigned long long done = 0;
     if (const int rc = opt_in(visc_face_rows8<NB, NQF, CONV, W>, smem, done)) return rc;
-    if (a.f.ngroups > 0) visc_face_rows8<NB, NQF, CONV, W><<<std::min(a.f.ngroups, sms), W * 32, smem, s>>>(a);
-    return cuda_status(cudaGetLastError());
+    return a.f.ngroups > 0 ? launch_early(visc_face_rows8<NB, NQF, CONV, W>, std::min(a.f.ngroups, sms), W * 32, smem, s, a) : (int)DG_OK;
 }
 
 template <int NB, int NQV, bool CONV>
@@ -36,8 +35,7 @@ int run_element(int sms, const Visc8Args& a, cudaStream_t s) {
     constexpr size_t smem = sizeof(ElemSmem8<NB>) * W;
     static unsigned long long done = 0;
     if (const int rc = opt_in(visc_element_rows8<NB, NQV, CONV, W>, smem, done)) return rc;
-    if (a.e.ngroups > 0) visc_element_rows8<NB, NQV, CONV, W><<<std::min(a.e.ngroups, sms), W * 32, smem, s>>>(a);
-    return cuda_status(cudaGetLastError());
+    return a.e.ngroups > 0 ? launch_early(visc_element_rows8<NB, NQV, CONV, W>, std::min(a.e.ngroups, sms), W * 32, smem, s, a) : (int)DG_OK;
 }
 
 }  // namespace

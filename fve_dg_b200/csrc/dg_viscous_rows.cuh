@@ -270,8 +270,10 @@ __global__ void __launch_bounds__(WARPS * 32, 1) visc_face_rows8(Visc8Args A) {
     if (lane == 0) mbar_init(&bars[warp], 16);
     __syncwarp();
     unsigned parity = 0;
-    for (int gi = blockIdx.x + gridDim.x * warp; gi < A.f.ngroups; gi += gridDim.x * WARPS)
+    for (int gi = blockIdx.x + gridDim.x * warp + await_previous(); gi < A.f.ngroups; gi += gridDim.x * WARPS) {
+        if (gi + gridDim.x * WARPS >= A.f.ngroups) release_next();
         if (!visc_face_group8<NB, NQF, CONV>(A, gi, sm, bars[warp], parity, lane)) break;
+    }
 }
 
 template <int NB, int NQV, bool CONV>
@@ -446,8 +448,10 @@ __global__ void __launch_bounds__(WARPS * 32, 1) visc_element_rows8(Visc8Args A)
     if (lane == 0) mbar_init(&bars[warp], 16);
     __syncwarp();
     unsigned parity = 0;
-    for (int gi = blockIdx.x + gridDim.x * warp; gi < A.e.ngroups; gi += gridDim.x * WARPS)
+    for (int gi = blockIdx.x + gridDim.x * warp + await_previous(); gi < A.e.ngroups; gi += gridDim.x * WARPS) {
+        if (gi + gridDim.x * WARPS >= A.e.ngroups) release_next();
         if (!visc_element_group8<NB, NQV, CONV>(A, gi, sm, bars[warp], parity, lane)) break;
+    }
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
