@@ -765,7 +765,7 @@ dg_ctx* create_impl(const dg_mesh_desc* mesh, const dg_config* cfg, int* err, co
                                       ? (size_t)c->nface * nqf * 5 : 0)) ||
         (rc = dev_alloc(&c->d_Un, nstate)) ||
         (rc = dev_alloc(&c->d_Ua, nstate)) || (rc = dev_alloc(&c->d_Ub, nstate)) ||
-        (rc = dev_alloc(&c->d_red, (size_t)kRedBlocks * 8)) || (rc = dev_alloc(&c->d_red_out, 8)))
+        (rc = dev_alloc(&c->d_red, (size_t)kRedMaxBlocks * 8)) || (rc = dev_alloc(&c->d_red_out, 8)))
         return fail(c, rc);
     if (inst_off && inst_off->size() >= 2) {
         c->ninst = (int)inst_off->size() - 1;
@@ -1526,7 +1526,7 @@ int dg_conservation(dg_ctx* c, double out[6]) {
     if (!c || !out) return DG_E_ARG;
     if (!c->have_state) return DG_E_STATE;
     DG_CUDA(cudaSetDevice(c->cfg.device));
-    return reduce_conservation(c->d_Un, c->d_geo, c->d_phi_v, c->d_w_v, (int)c->nowned, c->tab.nb, c->tab.nqv,
+    return reduce_conservation(c->d_Un, c->d_geo, c->d_phi_v, c->d_w_v, (int)c->nowned, c->tab.nb, c->tab.nqv, c->sms,
                                c->d_red, out, c->stream, &g_launches);
 }
 
@@ -1534,7 +1534,7 @@ int dg_max_wave_speed(dg_ctx* c, double* lam) {
     if (!c || !lam) return DG_E_ARG;
     if (!c->have_state) return DG_E_STATE;
     DG_CUDA(cudaSetDevice(c->cfg.device));
-    return reduce_wave_speed(c->d_Un, c->d_phi_v, (int)c->nowned, c->tab.nb, c->tab.nqv, c->cfg.gamma, c->d_red,
+    return reduce_wave_speed(c->d_Un, c->d_phi_v, (int)c->nowned, c->tab.nb, c->tab.nqv, c->cfg.gamma, c->sms, c->d_red,
                              lam, c->stream, &g_launches);
 }
 
@@ -1543,7 +1543,7 @@ int dg_check_state(dg_ctx* c, int64_t* bad) {
     if (!c->have_state) return DG_E_STATE;
     DG_CUDA(cudaSetDevice(c->cfg.device));
     double nbad = 0;
-    int rc = reduce_bad_points(c->d_Un, c->d_phi_v, (int)c->nowned, c->tab.nb, c->tab.nqv, c->cfg.gamma, c->d_red,
+    int rc = reduce_bad_points(c->d_Un, c->d_phi_v, (int)c->nowned, c->tab.nb, c->tab.nqv, c->cfg.gamma, c->sms, c->d_red,
                                &nbad, c->stream, &g_launches);
     if (rc) return rc;
     if (bad) *bad = (int64_t)nbad;
