@@ -25,6 +25,7 @@
 #include <cfloat>
 
 #include "dg_kernels_fp64.cuh"
+#include "dg_launch.cuh"
 #include "dg_status.cuh"
 #include "dg_mixed_host.cuh"
 
@@ -52,8 +53,21 @@ __device__ __forceinline__ double limiter_pressure(const double U[5], double gam
     return (gamma - 1.0) * (U[4] - ke);
 }
 
-constexpr int kLimWarps = 4;
-constexpr int kLimMaxPts = 64;  // volume points a warp holds, two per lane (the largest rule has 57)
+// limiter_pressure(U, gamma) < 0, without the division where the sign is clear of rounding: E (2 rho) against m^2,
+// a hundred units in the last place apart, and nothing near underflow.
+__device__ __forceinline__ bool negative_pressure(const double U[5], double gamma) {
+    const double rho = U[0];
+    if (rho <= 1e-16) return true;
+    const double m2 = U[1] * U[1] + U[2] * U[2] + U[3] * U[3], t = U[4] * (2.0 * rho);
+    if (gamma > 1.001) {
+        if (t > m2 * (1.0 + 1e-14) && t > 1e-80) return false;
+        if (t < m2 * (1.0 - 1e-14) && m2 > 1e-100 && rho < 1e100) return true;
+    }
+    return limiter_pressure(U, gamma) < 0;
+}
+
+constexpr int kLimWarps = 4;       // statistics alone
+constexpr int kLimApplyWarps = 8;  // the three steps, two blocks per SM
 
 // The volume rule's basis values transposed to [l][g] in shared memory: lanes over points read
 // consecutive doubles (conflict-free) for every mode l.
@@ -80,10 +94,11 @@ __device__ __forceinline__ void point_values_t(const double* sphi, const double*
 }
 
 // Lanes per cell in the apply pass: the cells of a warp are processed side by side by groups of G
-// lanes (G a power of two), each lane holding ceil(NQV / G) points.
+// lanes (G a power of two), each lane holding ceil(NQV / G) points. Few lanes: what a cell's lanes do alike (bounds,
+// reductions) is then shared by more cells of a warp instruction; as many as keep the points in registers.
 template <int NQV>
 struct LimGroup {
-    static constexpr int G = NQV <= 4 ? 4 : NQV <= 24 ? 8 : NQV <= 48 ? 16 : 32;
+    static constexpr int G = NQV <= 24 ? 4 : NQV <= 48 ? 8 : 16;
 };
 
 template <int G>
@@ -98,22 +113,21 @@ __device__ __forceinline__ double group_min(double v, unsigned mask) {
     for (int o = G / 2; o > 0; o >>= 1) v = ref_min(v, __shfl_xor_sync(mask, v, o));
     return v;
 }
-__device__ __forceinline__ bool group_any(bool p, unsigned mask) { return (__ballot_sync(mask, p) & mask) != 0u; }
 
 // A cell's statistics from its point values v[PPL][5], held by a group of G lanes (lane gl holds
 // points gl + G r): the max over the points of each variable and the values at the last point
 // (with only_avg: the mean, twice).
 template <int NQV, int G, int PPL>
 __device__ __forceinline__ void write_stats(const double (&v)[PPL][5], const double (&avg)[5], int gl, unsigned mask,
-                                            int only_avg, double* __restrict__ out) {
+                                            int only_avg, double* out, bool live = true) {
     if (only_avg) {
         #pragma unroll
         for (int k = 0; k < 5; ++k)
-            if (gl == k % G) { out[k] = avg[k]; out[5 + k] = avg[k]; }
+            if (live && gl == k % G) { out[k] = avg[k]; out[5 + k] = avg[k]; }
         return;
     }
     constexpr int LR = (NQV - 1) / G, LL = (NQV - 1) % G;
-    if (gl == LL) {
+    if (live && gl == LL) {
         #pragma unroll
         for (int k = 0; k < 5; ++k) out[5 + k] = v[LR][k];
     }
@@ -124,7 +138,7 @@ __device__ __forceinline__ void write_stats(const double (&v)[PPL][5], const dou
         for (int r = 0; r < PPL; ++r)
             if (gl + G * r < NQV) mx = ref_max(mx, v[r][k]);
         mx = group_max<G>(mx, mask);
-        if (gl == 0) out[k] = mx;
+        if (live && gl == 0) out[k] = mx;
     }
 }
 
@@ -163,170 +177,270 @@ __global__ void __launch_bounds__(kLimWarps * 32)
     }
 }
 
+// Shared memory of limiter_apply: the basis [mode][point], padded to G lanes x PPL points with zeros; per warp two
+// buffers of its cells' rows, and the scales of its cells' variables.
+template <int NB, int NQV>
+struct LimSizes {
+    static constexpr int G = LimGroup<NQV>::G, CPW = 32 / G, PPL = (NQV + G - 1) / G, GP = G * PPL;
+    static constexpr int CHUNK = CPW * 5 * NB;  // doubles
+    static constexpr size_t smem = sizeof(double) * (NB * GP + (kLimApplyWarps * (2 * CHUNK + CPW * 6)));
+};
+
+// (avg - min_b) / (avg - v_min + 1e-32) and its counterpart, at most 1 (PositiveLimiter.h:140-160)
+__device__ __forceinline__ double limiter_theta(double avg, double vmin, double vmax, double bmin, double bmax) {
+    const double tmin = (avg != vmin) ? (avg - bmin) / (avg - vmin + 1e-32) : 0.0;
+    const double tmax = (avg != vmax) ? (bmax - avg) / (vmax - avg + 1e-32) : 0.0;
+    return ref_min(ref_min(tmin, tmax), 1.0);
+}
+
 // The three steps per element (PositiveLimiter.h:128-258) for cells [0, ncell), CPW = 32 / G cells
 // per warp side by side (lanes over the points of their cell). Bounds: the max of the statistics'
 // maxima and the min of their last-point values over the cell and its face neighbours (nbr
 // [ncell][4], the cell itself across a boundary face), which is the max/min over the cell's faces of
-// the face bounds. Point values are evaluated once; after a step scales the modes l >= 1 of a
-// variable by theta, its point values become avg + theta (v - avg) (phi_0 = 1), which is what the
-// reference re-evaluates. A step whose test passes at every point costs one vote. stats_out: when
-// non-null, the statistics of the limited state (as
-// limiter_cell_stats computes them: re-evaluated from the new coefficients where the limiter acted),
-// the next stage's bounds.
+// the face bounds: lane i of a cell loads neighbour i's. Point values are evaluated once; after a
+// step scales the modes l >= 1 of a variable by theta, its point values become avg + theta (v - avg)
+// (phi_0 = 1), which is what the reference re-evaluates. stats_out: when non-null, the statistics of
+// the limited state (as limiter_cell_stats computes them: re-evaluated from the new coefficients
+// where the limiter acted), the next stage's bounds.
+//
+// All lanes stay together: a lane group without a cell repeats the warp's last one and stores nothing. Bound by
+// instruction issue and the chains within a cell, so: rows arrive two groups of cells ahead, in one piece per
+// warp; reductions and divisions of the five variables run side by side, one variable's quotients per lane; the
+// sign of a pressure needs no division (negative_pressure), and a bisection ends when its interval stands still.
+// A density wave near vacuum, per launch: P2, 105,456 cells 75 -> 44 us (58 % of issue slots, was 42; 23 million warp
+// instructions, were 32) against eight lanes a cell without copies ahead; P1, 131,712 cells 77 -> 48, P3, 48,000 cells
+// 87 -> 64.
 template <int NB, int NQV>
-__global__ void __launch_bounds__(kLimWarps * 32)
-    limiter_apply(double* __restrict__ U, const int* __restrict__ nbr, const double* __restrict__ stats,
-                  const double* __restrict__ phi, int64_t ncell, double gamma, int only_avg,
-                  double* __restrict__ stats_out) {
-    constexpr int G = LimGroup<NQV>::G, CPW = 32 / G;
-    constexpr int PPL = (NQV + G - 1) / G;  // points per lane
-    static_assert(NQV <= kLimMaxPts, "volume rule too large");
-    __shared__ double sphi[NQV * NB];
-    __shared__ double scoef[kLimWarps][CPW * 5 * NB];
-    __shared__ double sbnd[kLimWarps][CPW][10];
-    load_phi_t<NB, NQV>(sphi, phi);
-    __syncthreads();
+__global__ void __launch_bounds__(kLimApplyWarps * 32, 2)
+    limiter_apply(double* U, const int* __restrict__ nbr, const double* stats, const double* __restrict__ phi, int64_t ncell,
+                  double gamma, int only_avg, double* stats_out) {
+    using Z = LimSizes<NB, NQV>;
+    constexpr int G = Z::G, CPW = Z::CPW, PPL = Z::PPL, GP = Z::GP, B5 = 5 * NB;
+    constexpr bool PADS = GP != NQV;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double* sphi = reinterpret_cast<double*>(smem_raw);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double* rows = sphi + NB * GP + w * (2 * Z::CHUNK + CPW * 6);
+    double* scale = rows + 2 * Z::CHUNK;  // [cell][5 variables, 1 where any is to be stored]
+    for (int i = threadIdx.x; i < NB * GP; i += blockDim.x) {
+        const int l = i / GP, g = i - l * GP;
+        sphi[i] = g < NQV ? phi[g * NB + l] : 0.0;
+    }
+    __syncthreads();
     const int grp = lane / G, gl = lane - grp * G;
-    const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (grp * G));
-    double* u = scoef[w] + grp * (5 * NB);
-    double* bnd = sbnd[w][grp];
-    for (int64_t e0 = ((int64_t)blockIdx.x * kLimWarps + w) * CPW; e0 < ncell;
-         e0 += (int64_t)gridDim.x * kLimWarps * CPW) {
-        const int nc = (int)(ncell - e0 < CPW ? ncell - e0 : CPW);
-        {   // the next iteration's cells into L2 while these are limited
-            const int64_t en = e0 + (int64_t)gridDim.x * kLimWarps * CPW;
-            if (en < ncell) {
-                const int64_t bytes = (ncell - en < CPW ? ncell - en : CPW) * (5 * NB * 8);
-                for (int64_t off = (int64_t)lane * 128; off < bytes; off += 32 * 128)
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(U + en * (5 * NB)) + off));
+    const int64_t step = (int64_t)gridDim.x * kLimApplyWarps * CPW;
+    const bool pairs = (reinterpret_cast<uintptr_t>(U) & 15) == 0;
+    auto fetch = [&](int64_t e0, int buf) {
+        if (e0 < ncell) {
+            const double* from = U + e0 * B5;
+            const unsigned to = smem_addr(rows + buf * Z::CHUNK);
+            const int len = (int)(ncell - e0 < CPW ? ncell - e0 : CPW) * B5;
+            const int even = pairs ? len & ~1 : 0;
+            for (int i = 2 * lane; i < even; i += 64)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 8 * i), "l"(from + i) : "memory");
+            for (int i = even + lane; i < len; i += 32)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to + 8 * i), "l"(from + i) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto cell_of = [&](int64_t e0) { return e0 + grp < ncell ? e0 + grp : ncell - 1; };
+    int64_t e0 = ((int64_t)blockIdx.x * kLimApplyWarps + w) * CPW + await_previous();
+    int4 n4 = make_int4(0, 0, 0, 0);
+    if (e0 < ncell) n4 = __ldg(reinterpret_cast<const int4*>(nbr) + cell_of(e0));
+    fetch(e0, 0);
+    for (int buf = 0; e0 < ncell; e0 += step, buf ^= 1) {
+        const int64_t e = cell_of(e0);
+        const bool live = e0 + grp < ncell;
+        double* u = rows + buf * Z::CHUNK + (int)(e - e0) * B5;
+        // the bounds of neighbour gl (max, min per variable) and this lane's share of the cell's own
+        const int64_t nb_cell = (gl & 3) == 0 ? n4.x : (gl & 3) == 1 ? n4.y : (gl & 3) == 2 ? n4.z : n4.w;
+        double st[10], own[3];
+        #pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            const double2 x = __ldcg(reinterpret_cast<const double2*>(stats + nb_cell * 10) + i);
+            st[2 * i] = x.x;
+            st[2 * i + 1] = x.y;
+        }
+        #pragma unroll
+        for (int i = 0; i < 3; ++i) own[i] = __ldcg(stats + e * 10 + min((gl & 3) + 4 * i, 9));
+        if (e0 + step < ncell) n4 = __ldg(reinterpret_cast<const int4*>(nbr) + cell_of(e0 + step));
+        fetch(e0 + step, buf ^ 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        double v[PPL][5];
+        auto evaluate = [&]() {  // summed over the modes in order, as the reference evaluates a point value
+            #pragma unroll
+            for (int r = 0; r < PPL; ++r)
+                #pragma unroll
+                for (int k = 0; k < 5; ++k) v[r][k] = 0.0;
+            #pragma unroll 2
+            for (int l = 0; l < NB; ++l) {
+                double c[5];
+                #pragma unroll
+                for (int k = 0; k < 5; ++k) c[k] = u[5 * l + k];
+                #pragma unroll
+                for (int r = 0; r < PPL; ++r) {
+                    const double p = sphi[l * GP + gl + G * r];
+                    #pragma unroll
+                    for (int k = 0; k < 5; ++k) v[r][k] = fma(p, c[k], v[r][k]);
+                }
+            }
+        };
+        evaluate();
+        double avg[5];
+        #pragma unroll
+        for (int k = 0; k < 5; ++k) avg[k] = u[k];
+        if (PADS) {  // neutral in every step
+            #pragma unroll
+            for (int k = 0; k < 5; ++k)
+                if (gl + G * (PPL - 1) >= NQV) v[PPL - 1][k] = avg[k];
+        }
+        // the cell's bounds: max of maxima, min of last values. A NaN counts only where the cell's own value is
+        // one (the comparisons of the reference skip it elsewhere).
+        bool own_nan = false;
+        #pragma unroll
+        for (int i = 0; i < 10; ++i) {
+            if (st[i] != st[i]) st[i] = i < 5 ? -DBL_MAX : DBL_MAX;
+            const double o = own[i / 4];
+            if ((gl & 3) == i % 4) {
+                own_nan |= o != o;
+                st[i] = i < 5 ? ref_max(st[i], o) : ref_min(st[i], o);
+            }
+            #pragma unroll
+            for (int m = 2; m > 0; m >>= 1) {
+                const double other = __shfl_xor_sync(0xffffffffu, st[i], m);
+                st[i] = i < 5 ? ref_max(st[i], other) : ref_min(st[i], other);
             }
         }
-        const double* ug0 = U + e0 * (5 * NB);
-        for (int i = lane; i < nc * 5 * NB; i += 32) scoef[w][i] = ug0[i];  // the warp's cells, coalesced
-        __syncwarp();
-        if (grp < nc) {
-            const int64_t e = e0 + grp;
-            double* ug = U + e * (5 * NB);
-            for (int k = gl; k < 5; k += G) {  // the cell's bounds: max of maxima, min of last values
-                const int4 n = reinterpret_cast<const int4*>(nbr)[e];
-                const double* st = stats + k;
-                double bx = st[e * 10], bn = st[e * 10 + 5];
-                bx = ref_max(bx, st[(int64_t)n.x * 10]); bn = ref_min(bn, st[(int64_t)n.x * 10 + 5]);
-                bx = ref_max(bx, st[(int64_t)n.y * 10]); bn = ref_min(bn, st[(int64_t)n.y * 10 + 5]);
-                bx = ref_max(bx, st[(int64_t)n.z * 10]); bn = ref_min(bn, st[(int64_t)n.z * 10 + 5]);
-                bx = ref_max(bx, st[(int64_t)n.w * 10]); bn = ref_min(bn, st[(int64_t)n.w * 10 + 5]);
-                bnd[k] = bx;
-                bnd[5 + k] = bn;
-            }
-            __syncwarp(gmask);
-            double avg[5], v[PPL][5];
+        if (__any_sync(0xffffffffu, own_nan)) {
             #pragma unroll
-            for (int k = 0; k < 5; ++k) avg[k] = u[k];
-            #pragma unroll
-            for (int r = 0; r < PPL; ++r) {
-                const int g = gl + G * r;
-                if (g < NQV) point_values_t<NB, NQV>(sphi, u, g, v[r]);
-                else
-                    #pragma unroll
-                    for (int k = 0; k < 5; ++k) v[r][k] = avg[k];  // neutral for min/max and pressure
+            for (int i = 0; i < 10; ++i) {
+                const double o = __ldcg(stats + e * 10 + i);
+                if (o != o) st[i] = o;
             }
-            double s0 = 1.0, s1 = 1.0, s2 = 1.0, s3 = 1.0, s4 = 1.0;  // per-variable scale of modes l >= 1
-            bool changed = false;
-            // step 1: each variable within the cell's bounds
+        }
+        // step 1: each variable within the cell's bounds. Lane k of a cell forms the quotients of variable k,
+        // every lane those of the last one where a cell has four lanes.
+        unsigned acts = 0;
+        double qa = 0.0, qn = 0.0, qx = 0.0, qb = 0.0, qm = 0.0, last = 1.0;
+        double vmax[5];
+        #pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            double mn = DBL_MAX, mx = -DBL_MAX;
+            #pragma unroll
+            for (int r = 0; r < PPL; ++r)
+                if (gl + G * r < NQV) { mn = ref_min(mn, v[r][k]); mx = ref_max(mx, v[r][k]); }
+            mn = group_min<G>(mn, 0xffffffffu);
+            mx = group_max<G>(mx, 0xffffffffu);
+            vmax[k] = mx;
+            bool out = mn < st[5 + k] || mx > st[k];
+            if (PADS) out |= avg[k] < st[5 + k] || avg[k] > st[k];
+            if (out) acts |= 1u << k;
+            if (G > 4 || k < 4) {
+                if (gl == k) { qa = avg[k]; qn = mn; qx = mx; qb = st[5 + k]; qm = st[k]; }
+            } else {
+                last = limiter_theta(avg[k], mn, mx, st[5 + k], st[k]);
+            }
+        }
+        double s[5] = {1.0, 1.0, 1.0, 1.0, 1.0};  // per-variable scale of modes l >= 1
+        if (__any_sync(0xffffffffu, acts != 0u)) {
+            const double mine = limiter_theta(qa, qn, qx, qb, qm);
             #pragma unroll
             for (int k = 0; k < 5; ++k) {
-                const double bmax = bnd[k], bmin = bnd[5 + k];
-                bool out = false;
-                #pragma unroll
-                for (int r = 0; r < PPL; ++r) out |= (v[r][k] < bmin) | (v[r][k] > bmax);
-                if (!group_any(out, gmask)) continue;
-                double vmin = DBL_MAX, vmax = -DBL_MAX;
-                #pragma unroll
-                for (int r = 0; r < PPL; ++r)
-                    if (gl + G * r < NQV) { vmin = ref_min(vmin, v[r][k]); vmax = ref_max(vmax, v[r][k]); }
-                vmin = group_min<G>(vmin, gmask);
-                vmax = group_max<G>(vmax, gmask);
-                const double tmin = (avg[k] != vmin) ? (avg[k] - bmin) / (avg[k] - vmin + 1e-32) : 0.0;
-                const double tmax = (avg[k] != vmax) ? (bmax - avg[k]) / (vmax - avg[k] + 1e-32) : 0.0;
-                const double theta = ref_min(ref_min(tmin, tmax), 1.0);
-                if (k == 0) s0 *= theta;
-                else if (k == 1) s1 *= theta;
-                else if (k == 2) s2 *= theta;
-                else if (k == 3) s3 *= theta;
-                else s4 *= theta;
-                #pragma unroll
-                for (int r = 0; r < PPL; ++r) v[r][k] = avg[k] + theta * (v[r][k] - avg[k]);
-                changed = true;
-            }
-            // step 2: density at the points >= 1e-16
-            {
-                const double eps = 1e-16;
-                bool low = false;
-                #pragma unroll
-                for (int r = 0; r < PPL; ++r) low |= v[r][0] < eps;
-                if (group_any(low, gmask)) {
-                    double rmin = DBL_MAX;
+                const double theta = G > 4 || k < 4 ? __shfl_sync(0xffffffffu, mine, k, G) : last;
+                if (acts >> k & 1u) {
+                    s[k] = theta;
                     #pragma unroll
-                    for (int r = 0; r < PPL; ++r)
-                        if (gl + G * r < NQV) rmin = ref_min(rmin, v[r][0]);
-                    rmin = group_min<G>(rmin, gmask);
+                    for (int r = 0; r < PPL; ++r) v[r][k] = avg[k] + theta * (v[r][k] - avg[k]);
+                }
+            }
+        }
+        // step 2: density at the points >= 1e-16
+        {
+            const double eps = 1e-16;
+            double rmin = DBL_MAX;
+            bool low = false;
+            #pragma unroll
+            for (int r = 0; r < PPL; ++r) {
+                low |= v[r][0] < eps;
+                if (gl + G * r < NQV) rmin = ref_min(rmin, v[r][0]);
+            }
+            if (__any_sync(0xffffffffu, low)) {
+                rmin = group_min<G>(rmin, 0xffffffffu);
+                if (__ballot_sync(0xffffffffu, low) >> (lane - gl) & ((1ull << G) - 1)) {
                     const double eff = ref_max(avg[0], eps);
                     const double num = eff - eps, den = eff - rmin;
                     const double theta = (den < 1e-32) ? 0.0 : ref_min(1.0, num / den);
-                    s0 *= theta;
+                    s[0] *= theta;
                     #pragma unroll
                     for (int r = 0; r < PPL; ++r) v[r][0] = avg[0] + theta * (v[r][0] - avg[0]);
-                    changed = true;
+                    acts |= 1u;
                 }
             }
-            // step 3: pressure at the points >= 0 by bisection toward the mean
-            double tp = 1.0;
-            bool neg = false;
-            #pragma unroll
-            for (int r = 0; r < PPL; ++r) neg |= (gl + G * r < NQV) && limiter_pressure(v[r], gamma) < 0;
-            if (group_any(neg, gmask)) {
-                #pragma unroll
-                for (int r = 0; r < PPL; ++r) {
-                    if (gl + G * r >= NQV || limiter_pressure(v[r], gamma) >= 0) continue;
-                    double lo = 0.0, hi = 1.0, mid = 0.5 * (lo + hi);
-                    for (int it = 0; it < 100; ++it) {
-                        mid = 0.5 * (lo + hi);
-                        double um[5];
-                        #pragma unroll
-                        for (int k = 0; k < 5; ++k) um[k] = (1.0 - mid) * avg[k] + mid * v[r][k];
-                        if (limiter_pressure(um, gamma) < 0) hi = mid;
-                        else lo = mid;
-                    }
-                    tp = ref_min(tp, mid);
-                }
-                tp = group_min<G>(tp, gmask);
-                if (tp != 1.0) changed = true;
-            }
-            if (changed) {  // modes l >= 1: c *= theta_1 [*= theta_rho] *= theta_p, in the reference's order
-                __syncwarp(gmask);
-                for (int i = gl; i < 5 * (NB - 1); i += G) {
-                    const int k = i % 5;
-                    const double sk = k == 0 ? s0 : k == 1 ? s1 : k == 2 ? s2 : k == 3 ? s3 : s4;
-                    double c = u[5 + i];
-                    if (sk != 1.0) c *= sk;
-                    if (tp != 1.0) c *= tp;
-                    u[5 + i] = c;
-                    ug[5 + i] = c;
-                }
-                __syncwarp(gmask);
-                if (stats_out && !only_avg) {  // the limited state's point values, re-evaluated
-                    #pragma unroll
-                    for (int r = 0; r < PPL; ++r) {
-                        const int g = gl + G * r;
-                        if (g < NQV) point_values_t<NB, NQV>(sphi, u, g, v[r]);
-                    }
-                }
-            }
-            if (stats_out) write_stats<NQV, G, PPL>(v, avg, gl, gmask, only_avg, stats_out + e * 10);
         }
-        __syncwarp();
+        // step 3: pressure at the points >= 0 by bisection toward the mean
+        double tp = 1.0;
+        unsigned neg = 0;
+        #pragma unroll
+        for (int r = 0; r < PPL; ++r)
+            if (gl + G * r < NQV && negative_pressure(v[r], gamma)) neg |= 1u << r;
+        if (__any_sync(0xffffffffu, neg != 0u)) {
+            #pragma unroll
+            for (int r = 0; r < PPL; ++r) {
+                if (!(neg >> r & 1u)) continue;
+                double lo = 0.0, hi = 1.0, mid = 0.5 * (lo + hi);
+                for (int it = 0; it < 100; ++it) {
+                    mid = 0.5 * (lo + hi);
+                    double um[5];
+                    #pragma unroll
+                    for (int k = 0; k < 5; ++k) um[k] = (1.0 - mid) * avg[k] + mid * v[r][k];
+                    const bool low_side = negative_pressure(um, gamma);
+                    if (mid == (low_side ? hi : lo)) break;  // every further step would be the same
+                    if (low_side) hi = mid;
+                    else lo = mid;
+                }
+                tp = ref_min(tp, mid);
+            }
+            __syncwarp();
+            tp = group_min<G>(tp, 0xffffffffu);
+        }
+        const bool changed = acts != 0u || tp != 1.0;
+        if (__any_sync(0xffffffffu, changed)) {  // modes l >= 1: c *= theta_1 [*= theta_rho] *= theta_p, in the reference's order
+            if (gl == 0) {
+                #pragma unroll
+                for (int k = 0; k < 5; ++k) scale[grp * 6 + k] = s[k];
+            }
+            __syncwarp();
+            double* chunk = rows + buf * Z::CHUNK;
+            for (int i0 = 0; i0 < Z::CHUNK; i0 += 32) {
+                const int i = i0 + lane, c = min(i / B5, CPW - 1), rr = i - c * B5;
+                // the pressure scale and the flag are the cell's lanes': taken by shuffle
+                const double t = __shfl_sync(0xffffffffu, tp, c * G);
+                const bool act = __shfl_sync(0xffffffffu, (int)(changed && live), c * G);
+                if (act && i < Z::CHUNK && rr >= 5) {
+                    const double x = chunk[i] * scale[c * 6 + rr % 5] * t;
+                    chunk[i] = x;
+                    U[e0 * B5 + i] = x;
+                }
+            }
+            __syncwarp();
+            if (stats_out && !only_avg) {  // the limited state's point values, re-evaluated
+                evaluate();
+                write_stats<NQV, G, PPL>(v, avg, gl, 0xffffffffu, 0, stats_out + e * 10, live);
+            }
+        } else if (stats_out && !only_avg && live) {
+            constexpr int LR = (NQV - 1) / G, LL = (NQV - 1) % G;
+            #pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                if (gl == LL) stats_out[e * 10 + 5 + k] = v[LR][k];
+                if (gl == 0) stats_out[e * 10 + k] = vmax[k];
+            }
+        }
+        if (stats_out && only_avg) write_stats<NQV, G, PPL>(v, avg, gl, 0xffffffffu, 1, stats_out + e * 10, live);
+        __syncwarp();  // the buffer is free
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    release_next();
 }
 
 // X(order, qv, NB, NQV)
@@ -339,6 +453,18 @@ __global__ void __launch_bounds__(kLimWarps * 32)
     X(3, 4, 20, 31)             \
     X(4, 5, 35, 44)             \
     X(4, 6, 35, 57)
+
+template <int NB, int NQV>
+inline int run_limiter_apply(double* U, const int* nbr, const double* stats, const double* phi, int64_t ncell, double gamma,
+                             int only_avg, double* stats_out, int sms, cudaStream_t s) {
+    using Z = LimSizes<NB, NQV>;
+    static unsigned long long done = 0;
+    if (const int rc = ensure_smem(limiter_apply<NB, NQV>, Z::smem, done)) return rc;
+    const int64_t per_block = kLimApplyWarps * Z::CPW;
+    const int g = (int)std::max<int64_t>(1, std::min<int64_t>((ncell + per_block - 1) / per_block, 2 * (int64_t)sms));
+    return launch_early(limiter_apply<NB, NQV>, g, kLimApplyWarps * 32, Z::smem, s, U, nbr, stats, phi, ncell, gamma, only_avg,
+                        stats_out);
+}
 
 inline bool limiter_supported(int order, int qv) {
 #define X(P, QV, NB, NQV) \
@@ -357,9 +483,9 @@ inline int launch_limiter(int order, int qv, double* U, const double* Uprev, con
     if (order == P && qv == QV) {                                                                                \
         const unsigned ge = (unsigned)std::min<int64_t>((ncell + kLimWarps - 1) / kLimWarps, (int64_t)sms * 16); \
         limiter_cell_stats<NB, NQV><<<ge, kLimWarps * 32, 0, s>>>(Uprev, phi_v, 0, ncell, only_avg, stats);      \
-        limiter_apply<NB, NQV><<<ge, kLimWarps * 32, 0, s>>>(U, nbr, stats, phi_v, napply, gamma, only_avg,       \
-                                                             nullptr);                                           \
-        return cuda_status(cudaGetLastError());                                            \
+        const int rc = cuda_status(cudaGetLastError());                                                          \
+        if (rc) return rc;                                                                                       \
+        return run_limiter_apply<NB, NQV>(U, nbr, stats, phi_v, napply, gamma, only_avg, nullptr, sms, s);       \
     }
     FVEDG_LIMITER_COMBOS(X)
 #undef X
@@ -397,11 +523,8 @@ inline int launch_limiter_stage(int order, int qv, double* U, const double* Uin,
     if (rc) return rc;
 #define X(P, QV, NB, NQV)                                                                                         \
     if (order == P && qv == QV) {                                                                                 \
-        const unsigned ge = (unsigned)std::min<int64_t>((napply + kLimWarps - 1) / kLimWarps, (int64_t)sms * 16); \
-        limiter_apply<NB, NQV><<<ge, kLimWarps * 32, 0, s>>>(U, nbr, stats_in, phi_v, napply, gamma, only_avg,    \
-                                                             stats_out);                                          \
         ++*launches;                                                                                              \
-        return cuda_status(cudaGetLastError());                                             \
+        return run_limiter_apply<NB, NQV>(U, nbr, stats_in, phi_v, napply, gamma, only_avg, stats_out, sms, s);   \
     }
     FVEDG_LIMITER_COMBOS(X)
 #undef X
