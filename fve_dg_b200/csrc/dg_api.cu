@@ -20,6 +20,7 @@
 #include "dg_limiter.cuh"
 #include "dg_viscous.cuh"
 #include "dg_reduce.cuh"
+#include "dg_transfer.cuh"
 
 using namespace fvedg;
 
@@ -56,6 +57,7 @@ int upload(T** p, const std::vector<T>& v) {
 constexpr int kVisc8PerSm = 1;
 
 struct dg_ctx {
+    StageUse stage_use;
     dg_config cfg{};
     int qv = 0, qf = 0;
     int64_t ncell = 0, nface = 0;
@@ -589,6 +591,10 @@ int copy_in(dg_ctx* c, double* dev, const double* host, size_t stride, cudaStrea
     const size_t blk = sizeof(double) * 5 * c->tab.nb;
     if (stride == 0) stride = blk;
     if (stride < blk) return DG_E_ARG;
+    if (staged(host, blk, c->ncell)) {
+        const int rc = staged_copy(true, (char*)dev, (char*)host, stride, blk, c->ncell, c->cfg.device, s);
+        if (rc <= 0) return rc;
+    }
     if (stride == blk) return cuda_ok(cudaMemcpyAsync(dev, host, blk * c->ncell, cudaMemcpyHostToDevice, s));
     return cuda_ok(cudaMemcpy2DAsync(dev, blk, host, stride, blk, c->ncell, cudaMemcpyHostToDevice, s));
 }
@@ -596,6 +602,10 @@ int copy_out(dg_ctx* c, double* host, const double* dev, size_t stride, cudaStre
     const size_t blk = sizeof(double) * 5 * c->tab.nb;
     if (stride == 0) stride = blk;
     if (stride < blk) return DG_E_ARG;
+    if (staged(host, blk, c->ncell)) {
+        const int rc = staged_copy(false, (char*)dev, (char*)host, stride, blk, c->ncell, c->cfg.device, s);
+        if (rc <= 0) return rc;
+    }
     if (stride == blk) return cuda_ok(cudaMemcpyAsync(host, dev, blk * c->ncell, cudaMemcpyDeviceToHost, s));
     return cuda_ok(cudaMemcpy2DAsync(host, stride, dev, blk, blk, c->ncell, cudaMemcpyDeviceToHost, s));
 }
