@@ -20,6 +20,7 @@
 #include "dg_limiter.cuh"
 #include "dg_viscous.cuh"
 #include "dg_reduce.cuh"
+#include "dg_status_words.h"
 #include "dg_transfer.cuh"
 
 using namespace fvedg;
@@ -58,6 +59,7 @@ constexpr int kVisc8PerSm = 1;
 
 struct dg_ctx {
     StageUse stage_use;
+    int* status = nullptr;  // [kStatusWords] of the bounded waits
     dg_config cfg{};
     int qv = 0, qf = 0;
     int64_t ncell = 0, nface = 0;
@@ -567,19 +569,24 @@ int launches_per_step(const dg_ctx* c) {
     return 6 + lim;
 }
 
-// After a synchronize: the watchdog words of the persistent queue and of the mixed kernels' bounded
-// waits (DG_OK or DG_E_WATCHDOG); a set word is cleared.
+// After a synchronize: the status words of the kernels' bounded waits (DG_OK or DG_E_WATCHDOG), cleared. They lie in
+// mapped host memory: read by copies from the device they were 8 us of every stepping call.
+int check_status(dg_ctx* c) {
+    int rc = DG_OK;
+    for (int i = 0; i < kStatusWords; ++i) {
+        volatile int* word = c->status + i;
+        if (*word == DG_OK) continue;
+        *word = DG_OK;
+        rc = DG_E_WATCHDOG;
+    }
+    return rc;
+}
+
+// The same, and the word of the persistent queue.
 int check_queue(dg_ctx* c) {
     int err = 0;
-    for (int* word : {c->mixed.err, c->rows.err, c->visc8.own.err}) {
-        if (!word) continue;
-        if (cudaMemcpy(&err, word, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return DG_E_CUDA;
-        if (err != DG_OK) {
-            cudaMemset(word, 0, sizeof(int));
-            return DG_E_WATCHDOG;
-        }
-    }
-    if (!c->d_queue) return DG_OK;
+    if (const int rc = check_status(c)) return rc;
+    if (!c->d_queue || c->cfg.schedule != 1) return DG_OK;
     if (cudaMemcpy(&err, &c->d_queue->error, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return DG_E_CUDA;
     if (err == DG_OK) return DG_OK;
     cudaMemset(c->d_queue, 0, sizeof(QueueState));
@@ -638,6 +645,7 @@ void free_ctx(dg_ctx* c) {
                       c->d_visc_Av, c->d_visc_Pf, c->d_visc_vf, c->d_Rv})
         if (p) cudaFree(p);
     if (c->d_lim_prev) cudaFree(c->d_lim_prev);
+    if (c->status) StatusPages::get().give(c->status);
     if (c->d_elem_inst) cudaFree(c->d_elem_inst);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
@@ -759,6 +767,10 @@ dg_ctx* create_impl(const dg_mesh_desc* mesh, const dg_config* cfg, int* err, co
         if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
             c->sms = sms;
     }
+    if (!(c->status = StatusPages::get().take())) return fail(c, DG_E_NOMEM);
+    c->mixed.err = c->status;
+    c->rows.err = c->status + 1;
+    c->visc8.own.err = c->status + 2;
     std::vector<FaceGroup8> fg8;
     std::vector<ElemGroup8> eg8;
     const bool rows = cfg->precision == DG_PREC_FP64 &&
@@ -1002,8 +1014,8 @@ int dg_residual(dg_ctx* c, const double* U, double* R, size_t stride, double t, 
     if (!c->d_R && (rc = dev_alloc(&c->d_R, nstate))) return rc;
     if ((rc = copy_in(c, c->d_io, U, stride, c->stream))) return rc;
     if ((rc = dg_residual_device(c, c->d_io, c->d_R, t, part, c->stream))) return rc;
-    if ((rc = copy_out(c, R, c->d_R, stride, c->stream))) return rc;
-    return cuda_ok(cudaStreamSynchronize(c->stream));
+    if ((rc = copy_out(c, R, c->d_R, stride, c->stream)) || (rc = cuda_ok(cudaStreamSynchronize(c->stream)))) return rc;
+    return check_status(c);
 }
 
 int dg_viscous_residual_device(dg_ctx* c, const double* U, double* R, double mu, double prandtl, void* stream) {
@@ -1109,8 +1121,8 @@ int dg_viscous_residual(dg_ctx* c, const double* U, double* R, size_t stride, do
     if (!c->d_R && (rc = dev_alloc(&c->d_R, nstate))) return rc;
     if ((rc = copy_in(c, c->d_io, U, stride, c->stream))) return rc;
     if ((rc = dg_viscous_residual_device(c, c->d_io, c->d_R, mu, prandtl, c->stream))) return rc;
-    if ((rc = copy_out(c, R, c->d_R, stride, c->stream))) return rc;
-    return cuda_ok(cudaStreamSynchronize(c->stream));
+    if ((rc = copy_out(c, R, c->d_R, stride, c->stream)) || (rc = cuda_ok(cudaStreamSynchronize(c->stream)))) return rc;
+    return check_status(c);
 }
 
 int dg_limit_device(dg_ctx* c, double* U, const double* Uprev, int only_avg, void* stream) {

@@ -20,7 +20,7 @@ struct Rows8Data {
     const double* jd = nullptr;
     const double* inv_detj = nullptr;
     double* rec = nullptr;  // [nface][5][moment_row(nb)]
-    int* err = nullptr;
+    int* err = nullptr;  // status word in mapped host memory, the context's
 };
 
 inline bool rows8_supported(int order, int qv, int qf) {
@@ -56,6 +56,10 @@ inline bool rows8_groups(int order, int qv, int qf, int sms, const std::vector<F
                          std::vector<ElemGroup8>& eg, int per_sm) {
     if (!rows8_supported(order, qv, qf)) return false;
     if (nowned < (int64_t)per_sm * kRows8 * sms) return false;
+    // P4 has eight warps per SM: with the 44-point rule a second round of groups that is less than a fifth full costs
+    // more than it saves (10,368 cells: 283 us a step in threes, 298 in eights; 57 points: 354, 337)
+    const int64_t round = (int64_t)kRows8 * 8 * sms;
+    if (order == 4 && qv == 5 && per_sm > 0 && nowned > round && nowned * 5 < round * 6) return false;
     int inner = 0;
     build_groups(hfi, hef, nowned, fg, eg, &inner);
     return (int64_t)eg.size() * kRows8 * 3 <= nowned * 4 && (int64_t)fg.size() * kRows8 * 3 <= (int64_t)hfi.size() * 4;
@@ -122,14 +126,13 @@ inline int init_rows8(Rows8Data& m, const Tables& tab, const std::vector<double>
         (rc = rows8_upload(m, &m.inv_detj, inv_detj)) || (rc = rows8_upload(m, &m.fgroups, fg)) ||
         (rc = rows8_upload(m, &m.egroups, eg)))
         return rc;
-    for (int i = 0; i < 2; ++i) {
+    if (with_records) {
         void* p = nullptr;
-        const size_t n = i ? sizeof(int) : with_records ? sizeof(double) * nface * 5 * MR : 16;
+        const size_t n = sizeof(double) * nface * 5 * MR;
         if (cudaMalloc(&p, n) != cudaSuccess) return DG_E_NOMEM;
         m.bufs.push_back(p);
         if (cudaMemset(p, 0, n) != cudaSuccess) return DG_E_CUDA;
-        if (i) m.err = (int*)p;
-        else m.rec = (double*)p;
+        m.rec = (double*)p;
     }
     m.ready = true;
     return DG_OK;

@@ -153,7 +153,7 @@ struct MixedElemArgs {
     const double* dt_inst;   // optional per-instance time step (ensembles), indexed by elem_inst
     const int* elem_inst;    // [ncell] instance of each element
     const double* Rv;        // RK mode: viscous residual subtracted from R (Navier-Stokes), or null
-    int* err;                // device status word (DG_E_WATCHDOG when a bounded wait ran out), or null
+    int* err;                // status word in mapped host memory (DG_E_WATCHDOG when a bounded wait ran out), or null
 };
 
 // ---- MMA helpers ----------------------------------------------------------------------------------
@@ -815,7 +815,7 @@ __device__ __forceinline__ bool element_group_staged(const MixedElemArgs& a, int
         sm.sDT[lane] = dt * __ldg(a.inv_detj + e);
     }
     if (!mbar_wait_bounded(&st.bar, parity, kBulkSpinLimit)) {
-        if (lane == 0 && a.err) atomicExch(a.err, DG_E_WATCHDOG);
+        if (lane == 0 && a.err) *static_cast<volatile int*>(a.err) = DG_E_WATCHDOG;
         mbar_wait_bounded(&st.bar, parity, kBulkSpinLimit);  // copies in flight land before the warp leaves
         return false;
     }

@@ -80,7 +80,7 @@ struct Mixed16FaceArgs {
     int flux;
     int faces_mask;
     int vec;                 // all state rows start on 16-byte boundaries
-    int* err;                // device status word (DG_E_WATCHDOG when a bounded wait ran out), or null
+    int* err;                // status word in mapped host memory (DG_E_WATCHDOG when a bounded wait ran out), or null
 };
 
 struct Mixed16ElemArgs {

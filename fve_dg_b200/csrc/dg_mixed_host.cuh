@@ -38,7 +38,7 @@ struct MixedData {
     const double* dt_inst = nullptr;  // ensembles: per-instance dt (device), else null
     const int* elem_inst = nullptr;
     const double* Rv = nullptr;       // Navier-Stokes stepping: the stage input's viscous residual
-    int* err = nullptr;               // device status word of the mixed kernels (bounded waits)
+    int* err = nullptr;               // status word of the mixed kernels (bounded waits), in mapped host memory
     // element kernel: 0 = loads phase by phase (8-warp CTAs, four per SM), 2 = each group's rows
     // staged by TMA bulk copies (P1..P3, 16-byte aligned state buffers); chosen by dg_autotune
     int elem_kernel = 0;
@@ -284,12 +284,15 @@ inline int init_mixed16(MixedData& m, const Tables& tab, int64_t nface, int qf) 
 // Whether a mesh runs in groups of sixteen. One warp then holds five times the items of a group of three, so
 // there must be enough groups to fill the SMs several times over: measured per step against groups of three
 // (us, 6 n^3 tets), P1 86 -> 80 at n = 14 and 51 -> 63 at n = 11; P2 205 -> 202 at n = 18, 108 -> 124 at 14;
-// P3 174 -> 170 at n = 14, 100 -> 125 at 11; P4 184 -> 176 at n = 11, 90 -> 174 at 8. And the groups must be
+// P3 174 -> 170 at n = 14, 100 -> 125 at 11; P4 184 -> 176 at n = 11, 90 -> 174 at 8. From four groups per SM on a
+// scheduler has two P4 warps: 199 -> 222 at n = 12, 228 -> 226 at n = 13, so not between. And the groups must be
 // reasonably full: a mesh with many classes of face maps leaves the remainder of each class in a partial
 // group, which costs as much as a full one.
 inline bool wide_groups(MixedData& m, const std::vector<FaceInfo>& hfi, const std::vector<ElemFace>& hef, int64_t nowned) {
     const int64_t least = (int64_t)(m.order == 4 ? 3 : 10) * m.sms;
     if (nowned < least * kRows) return false;
+    const int64_t per_sm = (int64_t)kRows * m.sms;
+    if (m.order == 4 && nowned > 4 * per_sm && 2 * nowned < 11 * per_sm) return false;
     build_groups(hfi, hef, nowned, m.hfg16, m.heg16, &m.nfgroups_inner);
     if ((int64_t)m.heg16.size() * kRows * 3 <= nowned * 4 && (int64_t)m.hfg16.size() * kRows * 3 <= (int64_t)hfi.size() * 4)
         return true;
@@ -322,7 +325,7 @@ inline int init_mixed(MixedData& m, const Tables& tab, const std::vector<double>
     for (int g = 0; g < NQF; ++g) wsum += tab.w_f[g];
     m.t.wsum = wsum;
     int rc;
-    if ((rc = mixed_upload(m, &m.t.inv_mass, inv_mass)) || (rc = mixed_alloc(m, &m.err, 1))) return rc;
+    if ((rc = mixed_upload(m, &m.t.inv_mass, inv_mass))) return rc;
     m.wide = wide_groups(m, hfi, hef, nowned);
     if (m.wide) {
         if ((rc = init_mixed16(m, tab, nface, qf))) return rc;

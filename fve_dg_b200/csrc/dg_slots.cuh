@@ -54,7 +54,7 @@ struct RowSlotsOf {
 __device__ __forceinline__ bool rows_landed(uint64_t& bar, unsigned& parity, int* err, int lane) {
     bool ok = mbar_wait_bounded(&bar, parity, kBulkSpinLimit);
     if (!ok) {
-        if (lane == 0 && err) atomicExch(err, DG_E_WATCHDOG);
+        if (lane == 0 && err) *static_cast<volatile int*>(err) = DG_E_WATCHDOG;
         mbar_wait_bounded(&bar, parity, kBulkSpinLimit);
     }
     parity ^= 1u;
