@@ -147,8 +147,20 @@ def kernel_bytes(name, P, ncell, nface, nqf):
         return 3 * state + ncell * elem_rec + nface * nqf * 5 * 8
     if name == "limiter":                # bounds from the stage input, the output read and written
         return 3 * state + nface * (48 + 80) + ncell * 32
-    if name == "viscous":                # state read by both launches, residual written, face blocks
-        return 3 * state + 3 * nface * 8 * (5 * nqf + nb) + ncell * (80 + 8 + 32) + nface * 96
+    if name == "viscous":                # both launches of the operator: state read by each, residual written
+        return sum(kernel_bytes(k, P, ncell, nface, nqf) for k in ("visc_face_rows8", "visc_element_rows8")) - state
+    nm = {1: 1, 4: 3, 10: 6, 20: 10, 35: 15}.get(nb, 21)  # face flux moments of a variable
+    if name in ("face_flux_rows8", "element_rows8"):       # moments in whole 16-byte units, groups of eight
+        rec = nface * 5 * ((nm + 1) // 2 * 2) * 8
+        return state + nface * (face_rec + 6) + rec if name[0] == "f" else 3 * state + ncell * (80 + 24) + rec
+    if name in ("visc_face_rows8", "visc_element_rows8"):  # the same and the symmetric term per mode
+        rec = nface * (5 * ((nm + 1) // 2 * 2) + (nb + 1) // 2 * 2) * 8
+        return state + nface * (face_rec + 6) + rec + ncell * 88 if "face" in name else \
+            3 * state + ncell * (88 + 24) + rec
+    if name in ("face_flux_mixed16", "element_mixed16", "stage_persistent_mixed16"):  # groups of sixteen
+        rec = nface * 4 * (5 * ((max(nm, 3) + 4) // 8 * 8) + 20)
+        face, elem = state + nface * (face_rec + 5), 3 * state + ncell * (80 + 22)
+        return {"f": face + rec, "e": elem + rec, "s": face - state + elem + 2 * rec}[name[0]]
     kf = (nqf + 7) // 8 * 8
     fj = nface * (5 * kf * 4 + 2 * 5 * 8)  # face records: split flux deviations (A rows), FP64 reference, mode-0 sums
     grp = ncell * 96 // 3                  # element-group records
@@ -174,7 +186,7 @@ def algorithmic_bytes(name, P, ncell, nface, nqf):
         return state + 42 * nface
     if name.startswith("element"):
         return 3 * state + 80 * ncell
-    if name == "stage_persistent_mixed":
+    if name.startswith("stage_persistent"):
         return 3 * state + 80 * ncell + 42 * nface
     return kernel_bytes(name, P, ncell, nface, nqf)
 
@@ -384,7 +396,7 @@ def main():
 
     # per-kernel durations with CUDA events on the context stream (same workload, separate pass)
     kt = conv.ssprk3_timed(dt, args.steps)
-    roofline = make_roofline(kt, args.precision, schedule, P, m.ncell, m.nface, conv.nq_face, nb, args.config)
+    roofline = make_roofline(kt, args.precision, schedule, P, m.ncell, m.nface, conv.nq_face, nb, args.config, args.mu)
 
     # the other form on the same problem, same dt and steps from the same initial state
     forms = {args.precision: {"value": value, "ms_per_step": ms / args.steps, "schedule": schedule}}
@@ -398,10 +410,10 @@ def main():
         kt64 = f64.ssprk3_timed(dt, 3)
         forms["fp64"] = {"value": dof_stage_per_step * args.steps * world / (ms64 / 1e3),
                          "ms_per_step": ms64 / args.steps, "schedule": "two-launch",
-                         "kernels_ms_per_launch": {KNAMES[("fp64", "two-launch")].get(k, str(k)): v[0] / v[1]
+                         "kernels_ms_per_launch": {kernel_names("fp64", "two-launch", P, m.ncell, args.mu).get(k, str(k)): v[0] / v[1]
                                                    for k, v in kt64.items()},
                          "roofline": make_roofline(kt64, "fp64", "two-launch", P, m.ncell, m.nface, conv.nq_face, nb,
-                                                   args.config)}
+                                                   args.config, args.mu)}
         forms["mixed_over_fp64"] = forms["mixed"]["value"] / forms["fp64"]["value"]
         ctxs = {"mixed": conv, "fp64": f64}
         if schedule == "two-launch":
@@ -416,7 +428,7 @@ def main():
             ktb = bat.ssprk3_timed(dt, 3)
             vb = dof_stage_per_step * args.steps * world / (ms_b / 1e3)
             forms["mixed_batched"] = {"value": vb, "ms_per_step": ms_b / args.steps, "schedule": "persistent",
-                                      "kernels_ms_per_launch": {KNAMES[("mixed", "persistent")].get(k, str(k)):
+                                      "kernels_ms_per_launch": {kernel_names("mixed", "persistent", P, m.ncell).get(k, str(k)):
                                                                 v[0] / v[1] for k, v in ktb.items()}}
             forms["mixed_batched_over_fp64"] = vb / forms["fp64"]["value"]
             ctxs["mixed_batched"] = bat
@@ -506,9 +518,22 @@ def accuracy_report(ctxs, U0, dt, m, P, cfg, config, problems):
     return out
 
 
-KNAMES = {("fp64", "two-launch"): {0: "face_flux_tc", 1: "element_tc", 3: "viscous", 4: "limiter"},
-          ("mixed", "two-launch"): {0: "face_flux_mixed", 1: "element_mixed", 3: "viscous", 4: "limiter"},
-          ("mixed", "persistent"): {2: "stage_persistent_mixed", 3: "viscous", 4: "limiter"}}
+KNAMES = {("fp64", "two-launch"): {0: "face_flux_rows8", 1: "element_rows8", 3: "viscous", 4: "limiter"},
+          ("mixed", "two-launch"): {0: "face_flux_mixed16", 1: "element_mixed16", 3: "viscous", 4: "limiter"},
+          ("mixed", "persistent"): {2: "stage_persistent_mixed16", 3: "viscous", 4: "limiter"}}
+
+
+def kernel_names(precision, schedule, P, ncell, mu=0.0):
+    """Kernel per timing class: KNAMES, or on meshes too small for their groups the kernels for groups of three, and in
+    FP64 Navier-Stokes stepping the fused ones."""
+    names = dict(KNAMES[(precision, schedule)])
+    if precision == "fp64" and mu > 0:
+        names.update({0: "visc_face_rows8", 1: "visc_element_rows8"})
+    elif precision == "fp64" and ncell < 8 * 148 * (5 if P == 1 else 3):
+        names.update({0: "face_flux_tc", 1: "element_tc"})
+    elif precision == "mixed" and ncell < 16 * 148 * (3 if P == 4 else 10):
+        names = {k: v.removesuffix("16") for k, v in names.items()}
+    return names
 
 
 def time_steps(conv, dt, warmup, steps, dist, torch, launch_count):
@@ -559,14 +584,14 @@ def time_e2e(conv, dt, steps, dof_stage_per_step, world, dist, torch):
             "h2d_bytes_per_step": state_bytes, "d2h_bytes_per_step": state_bytes, "steps": k}
 
 
-def make_roofline(kt, precision, schedule, P, ncell, nface, nqf, nb, config):
+def make_roofline(kt, precision, schedule, P, ncell, nface, nqf, nb, config, mu=0.0):
     """Roofline object of the dominant kernel class of kt ({class: (total ms, launches)}): achieved GB/s
     on the algorithm's minimum bytes of one launch (algorithmic_bytes) over its average CUDA-event
     duration, against the measured HBM copy bandwidth. The bytes this implementation moves by design
     (its intermediates included) and the DRAM traffic ncu measured for the kernel are reported beside
     it, with their ratios to the algorithmic bytes. `stage` carries the stage-level figures on the
     algorithm's minimum bytes and flops per DOF-stage."""
-    names = KNAMES[(precision, schedule)]
+    names = kernel_names(precision, schedule, P, ncell, mu)
     peak, peak_kind = read_peaks()
     dom = max(kt, key=lambda k: kt[k][0])
     dom_ms = kt[dom][0] / kt[dom][1]
@@ -662,10 +687,7 @@ def run_viscous(args, cfg, rank, world, local, dist):
                              f"{kk} evaluations, {el:.1f} s", "cpu_model": cpu_model()}
     if rank == 0:
         ms_each = ms / args.steps
-        # the state read by both launches, the residual written, the per-face buffer written once and
-        # read from both sides, geometry and face records
-        face_block = 8 * (5 * conv.nq_face + nb)
-        bytes_each = 3 * dof * 8 + 3 * m.nface * face_block + m.ncell * (80 + 8 + 32) + m.nface * 48 * 2
+        bytes_each = kernel_bytes("viscous", P, m.ncell, m.nface, conv.nq_face)
         peak, peak_kind = read_peaks()
         traffic = None
         try:
@@ -680,12 +702,12 @@ def run_viscous(args, cfg, rank, world, local, dist):
                 "config": {"workload": args.config + "-viscous", "desc": cfg["desc"] + "; ExplicitDiffusion, mu = Pr = 1",
                            "tets": m.ncell, "order": P, "parallelism": f"independent instance per GPU x{world}"},
                 "gpu_launches": launches,
-                "roofline": {"bound": "hbm", "kernel": "viscous_face + viscous_element",
+                "roofline": {"bound": "hbm", "kernel": "visc_face_rows8 + visc_element_rows8",
                              "achieved": bytes_each / (ms_each / 1e3) / 1e9,
                              "peak": peak, "unit": "GB/s", "frac": bytes_each / (ms_each / 1e3) / 1e9 / peak,
                              "peak_kind": peak_kind, "traffic": traffic, "algorithmic_bytes_per_launch": bytes_each,
                              "note": "FP64 traces and contractions (on the FP64 tensor cores) per face and per "
-                                     "element: bound by instruction issue and latency, not by HBM"},
+                                     "element: bound by the FP64 pipe, not by HBM"},
                 "cpu_baseline": cpu,
                 "e2e": {"value": e2e, "unit": "DOF-residual/s", "h2d_bytes_per_step": dof * 8, "d2h_bytes_per_step": dof * 8,
                         "steps": k}}
@@ -941,7 +963,7 @@ def run_ensemble(args, rank, world, local, dist):
                           "batched_over_sequential": value / seq_value,
                           "l2_vs_fp64_max_over_instances": {"rho": float(max(e[0] for e in errs)),
                                                             "E": float(max(e[4] for e in errs))}},
-                "kernels_ms_per_launch": {KNAMES[("mixed", "persistent")].get(kk, str(kk)): v[0] / v[1]
+                "kernels_ms_per_launch": {kernel_names("mixed", "persistent", 2, ens.ncell).get(kk, str(kk)): v[0] / v[1]
                                           for kk, v in kt.items()},
                 "autotune": tune, "e2e": e2e, "clocks": clocks}
         print(json.dumps(line), flush=True)
