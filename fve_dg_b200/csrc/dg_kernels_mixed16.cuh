@@ -584,7 +584,7 @@ __device__ __forceinline__ bool element_group16(const Mixed16ElemArgs& a, const 
         if (lane < kRows) {  // the flux of the mean state, one lane per element
             const double* geo = sm.geo[lane];
             const double* row = a.U + mine * B5;
-            double c[5], J[9];
+            double c[5], J[9], Jf[9];
             #pragma unroll
             for (int i = 0; i < 5; ++i) c[i] = row[i];
             const double dj = geo[9];
@@ -594,22 +594,31 @@ __device__ __forceinline__ bool element_group16(const Mixed16ElemArgs& a, const 
             for (int i = 0; i < 9; ++i) {
                 J[i] = dj * geo[i];
                 sm.sJ[lane][i] = (float)J[i];
+                Jf[i] = (double)(float)J[i];
             }
             const double rho = c[0] > 1e-16 ? c[0] : 1e-16, ir = 1.0 / rho;
             const double u[3] = {c[1] * ir, c[2] * ir, c[3] * ir};
             const double p = (a.gamma - 1.0) * (c[4] - 0.5 * rho * (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]));
-            #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const double v = u[0] * J[d] + u[1] * J[3 + d] + u[2] * J[6 + d];
-                double g[5];
+            auto flux_d = [&](const double (&X)[9], int d, double (&g)[5]) {
+                const double v = u[0] * X[d] + u[1] * X[3 + d] + u[2] * X[6 + d];
                 g[0] = rho * v;
                 #pragma unroll
-                for (int i = 0; i < 3; ++i) g[1 + i] = rho * u[i] * v + p * J[3 * i + d];
+                for (int i = 0; i < 3; ++i) g[1 + i] = rho * u[i] * v + p * X[3 * i + d];
                 g[4] = (c[4] + p) * v;
+            };
+            // The points' fluxes are pulled back with the FP32 geometry, so the deviations are taken from the mean
+            // state's flux pulled back with it too; what that differs from its FP32 value goes to the FP64 part. With
+            // the exact flux rounded in its place every step had the same error of half an FP32 unit.
+            #pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                double g[5], gf[5];
+                flux_d(J, d, g);
+                flux_d(Jf, d, gf);
                 #pragma unroll
                 for (int k = 0; k < 5; ++k) {
-                    sm.sGb[lane][3 * k + d] = g[k];
-                    sm.sGbf[lane][3 * k + d] = (float)g[k];
+                    const float r = (float)gf[k];
+                    sm.sGb[lane][3 * k + d] = g[k] - (gf[k] - (double)r);
+                    sm.sGbf[lane][3 * k + d] = r;
                 }
             }
         }
@@ -637,7 +646,7 @@ __device__ __forceinline__ bool element_group16(const Mixed16ElemArgs& a, const 
         #pragma unroll 1
         for (int nt = 0; nt < MV / 8; ++nt) {
             // row r of the lane's pair: both its points at once
-            float2 U[5][2], np[2], v[3][2];
+            float2 U[5][2], np[2], mj[3][2], v[3][2];
             #pragma unroll
             for (int k = 0; k < 5; ++k) {
                 const float4 x = sm.val.v[k][nt][lane];
@@ -645,7 +654,9 @@ __device__ __forceinline__ bool element_group16(const Mixed16ElemArgs& a, const 
                 U[k][1] = make_float2(x.z, x.w);
             }
             // Gb - G per direction d: with v = u . J_d, G_0 = m . J_d, G_i = m_i v + p J_id, G_4 = (E + p) v;
-            // one variable at a time, directions 0 and 1 as one 16-wide k-tile, direction 2 as an 8-wide one
+            // one variable at a time, directions 0 and 1 as one 16-wide k-tile, direction 2 as an 8-wide one. The
+            // momentum's pressure comes last: taken from Gb first, it left a rounding that is the same at all points
+            // of a flow of one pressure, and 200 steps of a density wave (P2) were 20 % further off.
             #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 const float2 ir = rcp2(max2(U[0][r], 1e-16f));
@@ -658,8 +669,10 @@ __device__ __forceinline__ bool element_group16(const Mixed16ElemArgs& a, const 
                 np[r] = mul2(p, f2(-1.f));
                 const float* J = sm.sJ[gid + 8 * r];
                 #pragma unroll
-                for (int d = 0; d < 3; ++d)  // -v
-                    v[d][r] = fma2(vel[0], f2(-J[d]), fma2(vel[1], f2(-J[3 + d]), mul2(vel[2], f2(-J[6 + d]))));
+                for (int d = 0; d < 3; ++d) {  // -m . J_d, -v
+                    mj[d][r] = fma2(U[1][r], f2(-J[d]), fma2(U[2][r], f2(-J[3 + d]), mul2(U[3][r], f2(-J[6 + d]))));
+                    v[d][r] = mul2(mj[d][r], ir);
+                }
             }
             const uint32_t* tb = t.tvp + nt * NJ * VW;
             uint4 b01[NJ];
@@ -685,8 +698,8 @@ __device__ __forceinline__ bool element_group16(const Mixed16ElemArgs& a, const 
                             const float* J = sm.sJ[gid + 8 * r] + d;
                             const float2 gb = f2(sm.sGbf[gid + 8 * r][3 * k + d]);
                             float2 g;
-                            if (k == 0) g = fma2(U[1][r], f2(-J[0]), fma2(U[2][r], f2(-J[3]), fma2(U[3][r], f2(-J[6]), gb)));
-                            else if (k < 4) g = fma2(U[k][r], v[d][r], fma2(np[r], f2(J[3 * (k - 1)]), gb));
+                            if (k == 0) g = add2(gb, mj[d][r]);
+                            else if (k < 4) g = fma2(np[r], f2(J[3 * (k - 1)]), fma2(U[k][r], v[d][r], gb));
                             else g = fma2(U[4][r], v[d][r], gb);
                             split2(g.x, g.y, h[kk][2 * d + r], l[kk][2 * d + r]);
                         }
@@ -730,7 +743,11 @@ __device__ __forceinline__ bool element_group16(const Mixed16ElemArgs& a, const 
         }
     };
     if (a.mode != 0) fetch(0);
-    // face integrals of the moments m >= 3; side 1 negated exactly
+    // face integrals of the moments m >= 3; side 1 negated exactly. The tensor cores cut a sum to FP32 instead of
+    // rounding it, in proportion to what is in the accumulator already: at P2, where the errors add up the most, each
+    // face is summed by itself and added to the volume term by a rounding addition (density wave, 200 steps: 8 % less
+    // error; the kernel is no slower. At P3 and P4 it cost 0.7 % and the errors are below those of groups of three).
+    constexpr bool SUMS = NB == 10;
     if constexpr (KM > 0) {
         #pragma unroll 1
         for (int q = 0; q < 4; ++q) {
@@ -743,22 +760,29 @@ __device__ __forceinline__ bool element_group16(const Mixed16ElemArgs& a, const 
             const uint32_t* tb = t.tfl + (grp.meta[q] & 0xff) * NJ * KTiles<KM>::NT_U32;
             #pragma unroll
             for (int j = 0; j < NJ; ++j) {
+                float part[5][4] = {};
                 if constexpr (KM == 16) {
                     const uint4 b = tab4(tb + j * KTiles<KM>::NT_U32 + lane * 4);
                     #pragma unroll
-                    for (int k = 0; k < 5; ++k) mma16816(acc[k][j], F[k].h[0], b.x, b.y);
+                    for (int k = 0; k < 5; ++k) mma16816(SUMS ? part[k] : acc[k][j], F[k].h[0], b.x, b.y);
                     #pragma unroll
-                    for (int k = 0; k < 5; ++k) mma16816(acc[k][j], F[k].h[0], b.z, b.w);
+                    for (int k = 0; k < 5; ++k) mma16816(SUMS ? part[k] : acc[k][j], F[k].h[0], b.z, b.w);
                     #pragma unroll
-                    for (int k = 0; k < 5; ++k) mma16816(acc[k][j], F[k].l[0], b.x, b.y);
+                    for (int k = 0; k < 5; ++k) mma16816(SUMS ? part[k] : acc[k][j], F[k].l[0], b.x, b.y);
                 } else {
                     const uint2 b = tab2(tb + j * KTiles<KM>::NT_U32 + lane * 2);
                     #pragma unroll
-                    for (int k = 0; k < 5; ++k) mma1688(acc[k][j], F[k].th, b.x);
+                    for (int k = 0; k < 5; ++k) mma1688(SUMS ? part[k] : acc[k][j], F[k].th, b.x);
                     #pragma unroll
-                    for (int k = 0; k < 5; ++k) mma1688(acc[k][j], F[k].th, b.y);
+                    for (int k = 0; k < 5; ++k) mma1688(SUMS ? part[k] : acc[k][j], F[k].th, b.y);
                     #pragma unroll
-                    for (int k = 0; k < 5; ++k) mma1688(acc[k][j], F[k].tl, b.x);
+                    for (int k = 0; k < 5; ++k) mma1688(SUMS ? part[k] : acc[k][j], F[k].tl, b.x);
+                }
+                if (SUMS) {
+                    #pragma unroll
+                    for (int k = 0; k < 5; ++k)
+                        #pragma unroll
+                        for (int i = 0; i < 4; ++i) acc[k][j][i] += part[k][i];
                 }
             }
         }
