@@ -103,6 +103,15 @@ inline int init_rows8(Rows8Data& m, const Tables& tab, const std::vector<double>
                         const int g = 8 * nt + 2 * (l % 4) + i, b = 8 * j + l / 4;
                         tw.push_back(g < NQV && b < NB ? tab.dphi_vw[((size_t)g * NB + b) * 3 + d] : 0.0);
                     }
+    std::vector<double> mv;
+    for (int j = 0; j < NJ; ++j)
+        for (int l = 0; l < 32; ++l) {
+            const int b = 8 * j + l / 4, d = l % 4;
+            long double s = 0;
+            if (b < NB && d < 3)
+                for (int g = 0; g < NQV; ++g) s -= tab.dphi_vw[((size_t)g * NB + b) * 3 + d];
+            mv.push_back((double)s);
+        }
     for (int p = 0; p < 24; ++p)
         for (int t = 0; t < KF; ++t)
             for (int j = 0; j < NJ; ++j)
@@ -122,7 +131,7 @@ inline int init_rows8(Rows8Data& m, const Tables& tab, const std::vector<double>
     int rc;
     if ((rc = rows8_upload(m, &m.t.tf, tf)) || (rc = rows8_upload(m, &m.t.tm, tm)) || (rc = rows8_upload(m, &m.t.tv, tv)) ||
         (rc = rows8_upload(m, &m.t.tw, tw)) || (rc = rows8_upload(m, &m.t.tl, tl)) ||
-        (rc = rows8_upload(m, &m.t.inv_mass, inv_mass)) || (rc = rows8_upload(m, &m.jd, jd)) ||
+        (rc = rows8_upload(m, &m.t.mv, mv)) || (rc = rows8_upload(m, &m.t.inv_mass, inv_mass)) || (rc = rows8_upload(m, &m.jd, jd)) ||
         (rc = rows8_upload(m, &m.inv_detj, inv_detj)) || (rc = rows8_upload(m, &m.fgroups, fg)) ||
         (rc = rows8_upload(m, &m.egroups, eg)))
         return rc;
