@@ -396,7 +396,8 @@ def main():
 
     # per-kernel durations with CUDA events on the context stream (same workload, separate pass)
     kt = conv.ssprk3_timed(dt, args.steps)
-    roofline = make_roofline(kt, args.precision, schedule, P, m.ncell, m.nface, conv.nq_face, nb, args.config, args.mu)
+    roofline = make_roofline(kt, args.precision, schedule, P, m.ncell, m.nface, conv.nq_face, nb, args.config, args.mu,
+                             conv)
 
     # the other form on the same problem, same dt and steps from the same initial state
     forms = {args.precision: {"value": value, "ms_per_step": ms / args.steps, "schedule": schedule}}
@@ -410,10 +411,10 @@ def main():
         kt64 = f64.ssprk3_timed(dt, 3)
         forms["fp64"] = {"value": dof_stage_per_step * args.steps * world / (ms64 / 1e3),
                          "ms_per_step": ms64 / args.steps, "schedule": "two-launch",
-                         "kernels_ms_per_launch": {kernel_names("fp64", "two-launch", P, m.ncell, args.mu).get(k, str(k)): v[0] / v[1]
+                         "kernels_ms_per_launch": {kernel_names("fp64", "two-launch", f64, args.mu).get(k, str(k)): v[0] / v[1]
                                                    for k, v in kt64.items()},
                          "roofline": make_roofline(kt64, "fp64", "two-launch", P, m.ncell, m.nface, conv.nq_face, nb,
-                                                   args.config, args.mu)}
+                                                   args.config, args.mu, f64)}
         forms["mixed_over_fp64"] = forms["mixed"]["value"] / forms["fp64"]["value"]
         ctxs = {"mixed": conv, "fp64": f64}
         if schedule == "two-launch":
@@ -428,7 +429,7 @@ def main():
             ktb = bat.ssprk3_timed(dt, 3)
             vb = dof_stage_per_step * args.steps * world / (ms_b / 1e3)
             forms["mixed_batched"] = {"value": vb, "ms_per_step": ms_b / args.steps, "schedule": "persistent",
-                                      "kernels_ms_per_launch": {kernel_names("mixed", "persistent", P, m.ncell).get(k, str(k)):
+                                      "kernels_ms_per_launch": {kernel_names("mixed", "persistent", bat).get(k, str(k)):
                                                                 v[0] / v[1] for k, v in ktb.items()}}
             forms["mixed_batched_over_fp64"] = vb / forms["fp64"]["value"]
             ctxs["mixed_batched"] = bat
@@ -523,15 +524,16 @@ KNAMES = {("fp64", "two-launch"): {0: "face_flux_rows8", 1: "element_rows8", 3: 
           ("mixed", "persistent"): {2: "stage_persistent_mixed16", 3: "viscous", 4: "limiter"}}
 
 
-def kernel_names(precision, schedule, P, ncell, mu=0.0):
-    """Kernel per timing class: KNAMES, or on meshes too small for their groups the kernels for groups of three, and in
-    FP64 Navier-Stokes stepping the fused ones."""
+def kernel_names(precision, schedule, conv=None, mu=0.0):
+    """Kernel per timing class: KNAMES (those of large meshes), or what the context says that it takes; in FP64
+    Navier-Stokes stepping the fused ones."""
     names = dict(KNAMES[(precision, schedule)])
-    if precision == "fp64" and mu > 0:
+    group = conv.kernel_group() if conv is not None else 0
+    if precision == "fp64" and mu > 0 and (conv is None or conv.kernel_group(viscous=True) == 8):
         names.update({0: "visc_face_rows8", 1: "visc_element_rows8"})
-    elif precision == "fp64" and ncell < 8 * 148 * (5 if P == 1 else 3):
-        names.update({0: "face_flux_tc", 1: "element_tc"})
-    elif precision == "mixed" and ncell < 16 * 148 * (3 if P == 4 else 10):
+    elif precision == "fp64" and group in (1, 3):
+        names.update({0: "face_flux_tc", 1: "element_tc"} if group == 3 else {0: "face_flux_fp64", 1: "element_fp64"})
+    elif precision == "mixed" and group == 3:
         names = {k: v.removesuffix("16") for k, v in names.items()}
     return names
 
@@ -584,14 +586,14 @@ def time_e2e(conv, dt, steps, dof_stage_per_step, world, dist, torch):
             "h2d_bytes_per_step": state_bytes, "d2h_bytes_per_step": state_bytes, "steps": k}
 
 
-def make_roofline(kt, precision, schedule, P, ncell, nface, nqf, nb, config, mu=0.0):
+def make_roofline(kt, precision, schedule, P, ncell, nface, nqf, nb, config, mu=0.0, conv=None):
     """Roofline object of the dominant kernel class of kt ({class: (total ms, launches)}): achieved GB/s
     on the algorithm's minimum bytes of one launch (algorithmic_bytes) over its average CUDA-event
     duration, against the measured HBM copy bandwidth. The bytes this implementation moves by design
     (its intermediates included) and the DRAM traffic ncu measured for the kernel are reported beside
     it, with their ratios to the algorithmic bytes. `stage` carries the stage-level figures on the
     algorithm's minimum bytes and flops per DOF-stage."""
-    names = kernel_names(precision, schedule, P, ncell, mu)
+    names = kernel_names(precision, schedule, conv, mu)
     peak, peak_kind = read_peaks()
     dom = max(kt, key=lambda k: kt[k][0])
     dom_ms = kt[dom][0] / kt[dom][1]
@@ -963,7 +965,7 @@ def run_ensemble(args, rank, world, local, dist):
                           "batched_over_sequential": value / seq_value,
                           "l2_vs_fp64_max_over_instances": {"rho": float(max(e[0] for e in errs)),
                                                             "E": float(max(e[4] for e in errs))}},
-                "kernels_ms_per_launch": {kernel_names("mixed", "persistent", 2, ens.ncell).get(kk, str(kk)): v[0] / v[1]
+                "kernels_ms_per_launch": {kernel_names("mixed", "persistent", ens).get(kk, str(kk)): v[0] / v[1]
                                           for kk, v in kt.items()},
                 "autotune": tune, "e2e": e2e, "clocks": clocks}
         print(json.dumps(line), flush=True)

@@ -67,6 +67,7 @@ def lib():
         "dg_residual_device": (ctypes.c_int, [vp, vp, vp, ctypes.c_double, ctypes.c_int, vp]),
         "dg_residual_device_static": (ctypes.c_int, [vp, vp, vp, ctypes.c_int, vp]),
         "dg_watchdog_selftest": (ctypes.c_int, [vp, ctypes.c_int64]),
+        "dg_kernel_group": (ctypes.c_int, [vp, ctypes.c_int]),
         "dg_last_cuda_error": (ctypes.c_char_p, []),
         "dg_static_scratch_capacity": (ctypes.c_int64, []),
         "dg_set_state": (ctypes.c_int, [vp, c_double_p, ctypes.c_size_t]),
@@ -137,7 +138,7 @@ def exported_symbols():
             "dg_refresh_split", "dg_ssprk3_stage", "dg_ssprk3_stage_phase", "dg_create_ensemble",
             "dg_ensemble_offsets", "dg_ssprk3_ensemble", "dg_autotune", "dg_set_element_shape", "dg_partition_create", "dg_partition_destroy",
             "dg_partition_local_mesh", "dg_partition_counts", "dg_partition_l2g", "dg_partition_global_faces",
-            "dg_partition_send", "dg_partition_recv", "dg_halo_pack", "dg_halo_unpack", "dg_watchdog_selftest", "dg_mass", "dg_limit", "dg_limit_device", "dg_viscous_residual", "dg_viscous_residual_device",
+            "dg_partition_send", "dg_partition_recv", "dg_halo_pack", "dg_halo_unpack", "dg_kernel_group", "dg_watchdog_selftest", "dg_mass", "dg_limit", "dg_limit_device", "dg_viscous_residual", "dg_viscous_residual_device",
             "dg_save_checkpoint", "dg_load_checkpoint",
             "dg_set_dirichlet", "dg_conservation",
             "dg_max_wave_speed", "dg_check_state", "dg_info", "dg_mesh_geometry", "dg_face_perms", "dg_basis",

@@ -119,6 +119,11 @@ class ExplicitConvection:
         """Pin the two-launch element kernel's shape (a choice dg_autotune records)."""
         L.check(L.lib().dg_set_element_shape(self._ctx, int(bool(staged)), int(ctas_per_sm)), "dg_set_element_shape")
 
+    def kernel_group(self, viscous=False):
+        """Items that a warp of this context's kernels (or its viscous ones) takes at a time: 16, 8, 3 or 1; 0 before
+        the viscous operator's first call."""
+        return L.lib().dg_kernel_group(self._ctx, int(bool(viscous)))
+
     def _state(self, U):
         U = L.as_f64(U)
         if U.shape != self.shape:

@@ -945,6 +945,13 @@ int dg_info(const dg_ctx* c, int* nb, int* nqv, int* nqf, int* qv, int* qf) {
     return DG_OK;
 }
 
+int dg_kernel_group(const dg_ctx* c, int viscous) {
+    if (!c) return DG_E_ARG;
+    if (viscous) return c->visc8.ready ? kRows8 : c->d_visc_vf ? 1 : 0;
+    if (c->cfg.precision == DG_PREC_MIXED) return c->mixed.wide ? kRows : 3;
+    return c->rows.ready ? kRows8 : c->tc.ready ? 3 : 1;
+}
+
 int dg_residual_device(dg_ctx* c, const double* U, double* R, double t, int part, void* stream) {
     (void)t;
     if (!c || !U || !R || part < 0 || part > 3) return DG_E_ARG;

@@ -195,6 +195,13 @@ int dg_autotune(dg_ctx* ctx, double dt, char* report, size_t len);
  * values, an FP64 context or a staged shape at order 4. New: no reference counterpart. */
 int dg_set_element_shape(dg_ctx* ctx, int staged, int ctas_per_sm);
 
+/* Items (faces or elements) that a warp of this context's kernels takes at a time, chosen from the mesh at creation:
+ * 16 (mixed form) or 8 (FP64) where there are enough groups of items with equal face maps and these are reasonably full,
+ * else 3, or 1 for the scalar FP64 kernels. viscous != 0: of the viscous operator, 8 or 1, and 0 before its first call
+ * (with mu > 0 there is none); with 8, an FP64 context with mu > 0 runs a Navier-Stokes stage as two fused launches.
+ * DG_E_ARG for a null context. New: no reference counterpart. */
+int dg_kernel_group(const dg_ctx* ctx, int viscous);
+
 /* Self-test of the failure detection of the batched persistent form (mixed precision, schedule 1):
  * runs stage 0 of one SSP-RK3 step with the completion count that face region 0 must reach raised
  * by one, so every wait of an element tile on that region runs out after `polls` polls (each about
