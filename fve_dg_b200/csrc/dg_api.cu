@@ -384,7 +384,7 @@ int viscous_buffers(dg_ctx* c) {
         return init_visc8(c->visc8, t, c->nface, c->qf);
     }
     const bool fused = c->cfg.mu > 0.0 && c->cfg.precision == DG_PREC_FP64;
-    if (c->cfg.order >= 1 && c->cfg.order <= 4 && rows8_supported(c->cfg.order, c->qv, c->qf)) {
+    if (c->cfg.order >= 1 && c->cfg.order <= 4 && (fused || c->nowned >= (int64_t)kVisc8PerSm * kRows8 * c->sms)) {
         std::vector<FaceInfo> hfi(c->nface);
         std::vector<ElemFace> hef(4 * c->ncell);
         std::vector<double> hgeo(10 * c->ncell);
@@ -392,7 +392,7 @@ int viscous_buffers(dg_ctx* c) {
         std::vector<ElemGroup8> eg;
         DG_CUDA(cudaMemcpy(hfi.data(), c->d_fi, sizeof(FaceInfo) * hfi.size(), cudaMemcpyDeviceToHost));
         DG_CUDA(cudaMemcpy(hef.data(), c->d_ef, sizeof(ElemFace) * hef.size(), cudaMemcpyDeviceToHost));
-        if (rows8_groups(c->cfg.order, c->qv, c->qf, c->sms, hfi, hef, c->nowned, fg, eg, fused ? 0 : kVisc8PerSm)) {
+        if (rows8_groups(c->cfg.order, c->qv, c->qf, hfi, hef, c->nowned, fg, eg)) {
             DG_CUDA(cudaMemcpy(hgeo.data(), c->d_geo, sizeof(double) * hgeo.size(), cudaMemcpyDeviceToHost));
             c->visc8.own.sms = c->sms;
             int rc = init_rows8(c->visc8.own, t, hgeo, fg, eg, c->ncell, c->nface, c->qv, c->qf, false);
@@ -774,7 +774,8 @@ dg_ctx* create_impl(const dg_mesh_desc* mesh, const dg_config* cfg, int* err, co
     std::vector<FaceGroup8> fg8;
     std::vector<ElemGroup8> eg8;
     const bool rows = cfg->precision == DG_PREC_FP64 &&
-                      rows8_groups(cfg->order, qv, qf, c->sms, hfi, hef, c->nowned, fg8, eg8, rows8_per_sm(cfg->order));
+                      rows8_convective(cfg->order, qv, c->nowned, c->sms) &&
+                      rows8_groups(cfg->order, qv, qf, hfi, hef, c->nowned, fg8, eg8);
     if ((rc = upload(&c->d_h, hh)) || (rc = upload(&c->d_dphi_v, c->tab.dphi_v)) ||
         (rc = upload(&c->d_dphi_f, c->tab.dphi_f)))
         return fail(c, rc);

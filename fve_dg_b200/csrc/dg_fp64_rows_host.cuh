@@ -42,24 +42,27 @@ inline int rows8_upload(Rows8Data& m, const T** dst, const std::vector<T>& v) {
     return DG_OK;
 }
 
-// Whether a mesh runs in rows of eight, with its groups. Orders 0 and 5 have no other tensor-core kernels and
-// always do (P0 56 -> 39 us a step at n = 4 against the runtime-size kernels, P5 326 -> 233; n = 24: 372 -> 260 and
-// 16,345 -> 4,838). For the others groups of three are the faster on small meshes, where a warp's chain of work
-// decides (us a step, three / eight: P1 31 / 36 at n = 8, 34 / 36 at n = 9, 42 / 40 at n = 11; P2 54 / 54 at n = 6,
-// 60 / 56 at n = 8, 64 / 58 at n = 9; P3 68 / 74, 80 / 79, 93 / 81; P4 103 / 127, 131 / 134, 177 / 140): five groups per
-// SM at P1, about 6,000 cells, three above. And the groups must be reasonably full (many classes of face maps leave
-// as many partial groups).
-inline int rows8_per_sm(int order) { return order == 0 || order == 5 ? 0 : order == 1 ? 5 : 3; }
-
-inline bool rows8_groups(int order, int qv, int qf, int sms, const std::vector<FaceInfo>& hfi,
-                         const std::vector<ElemFace>& hef, int64_t nowned, std::vector<FaceGroup8>& fg,
-                         std::vector<ElemGroup8>& eg, int per_sm) {
-    if (!rows8_supported(order, qv, qf)) return false;
+// Whether the convective operator of a mesh of that many cells runs in rows of eight. Orders 0 and 5 have no other
+// tensor-core kernels and take them at any size (P0 56 -> 39 us a step at n = 4 against the runtime-size kernels, P5
+// 326 -> 233; n = 24: 372 -> 260 and 16,345 -> 4,838). For the others groups of three are the faster on small meshes,
+// where a warp's chain of work decides (us a step, three / eight: P1 31 / 36 at n = 8, 34 / 36 at n = 9, 42 / 40 at
+// n = 11; P2 54 / 54 at n = 6, 60 / 56 at n = 8, 64 / 58 at n = 9; P3 68 / 74, 80 / 79, 93 / 81; P4 103 / 127, 131 / 134,
+// 177 / 140): five groups per SM at P1, about 6,000 cells, three above.
+inline bool rows8_convective(int order, int qv, int64_t nowned, int sms) {
+    const int per_sm = order == 0 || order == 5 ? 0 : order == 1 ? 5 : 3;
     if (nowned < (int64_t)per_sm * kRows8 * sms) return false;
     // P4 has eight warps per SM: with the 44-point rule a second round of groups that is less than a fifth full costs
     // more than it saves (10,368 cells: 283 us a step in threes, 298 in eights; 57 points: 354, 337)
     const int64_t round = (int64_t)kRows8 * 8 * sms;
-    if (order == 4 && qv == 5 && per_sm > 0 && nowned > round && nowned * 5 < round * 6) return false;
+    return !(order == 4 && qv == 5 && nowned > round && nowned * 5 < round * 6);
+}
+
+// The groups of eight, and whether they are full enough to use: a mesh with many classes of face maps (node orders of
+// cells and faces as another program lists them) leaves as many partial groups, each as costly as a full one, and takes
+// the other kernels at any size; orders 0 and 5 then take the scalar ones.
+inline bool rows8_groups(int order, int qv, int qf, const std::vector<FaceInfo>& hfi, const std::vector<ElemFace>& hef,
+                         int64_t nowned, std::vector<FaceGroup8>& fg, std::vector<ElemGroup8>& eg) {
+    if (!rows8_supported(order, qv, qf)) return false;
     int inner = 0;
     build_groups(hfi, hef, nowned, fg, eg, &inner);
     return (int64_t)eg.size() * kRows8 * 3 <= nowned * 4 && (int64_t)fg.size() * kRows8 * 3 <= (int64_t)hfi.size() * 4;

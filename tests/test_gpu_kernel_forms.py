@@ -158,3 +158,17 @@ def test_many_classes_of_face_maps_mixed():
         out.append(c.eval(U))
         c.close()
     assert rel_l2(out[1], out[0]) < RES_TOL
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_viscous_operator_between_the_convective_lines(precision):
+    """P4 with the 44-point rule at 10,368 cells: the convective kernels' line there is not the viscous ones'."""
+    m = box_mesh(12, jitter=0.1, seed=5)
+    U = state(m, 4)
+    out = []
+    for mu in (0.0, 0.3):  # mu > 0 in FP64: the fused kernels' groups, at any size
+        c = ExplicitConvection(m, order=4, quad_vol=5, quad_face=3, precision=precision, mu=mu)
+        out.append(c.viscous_eval(U, mu=0.3, prandtl=0.72))
+        assert c.kernel_group() == 3 and c.kernel_group(viscous=True) == 8
+        c.close()
+    assert np.array_equal(out[0], out[1])
