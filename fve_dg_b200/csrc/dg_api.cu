@@ -375,8 +375,9 @@ int timed(dg_ctx* c, int cls, cudaStream_t s, F&& fn) {
 // One SSP-RK3 step (Shu-Osher) on the device state, FP64 form:
 //   U1 = U + dt L(U);  U2 = 3/4 U + 1/4 (U1 + dt L(U1));  U = 1/3 U + 2/3 (U2 + dt L(U2)).
 // The viscous operator's tables (the volume ones transposed so that lanes over points read rows,
-// the A operands of its tensor-core products) and its per-face buffer; made by the first call.
-int viscous_buffers(dg_ctx* c) {
+// the A operands of its tensor-core products) and its per-face buffer; made by the first call, or at creation, which has
+// the face and element lists at hand.
+int viscous_buffers(dg_ctx* c, const std::vector<FaceInfo>* faces = nullptr, const std::vector<ElemFace>* elems = nullptr) {
     if (c->d_visc_vf || c->visc8.ready) return DG_OK;
     const Tables& t = c->tab;
     if (c->cfg.order >= 1 && c->cfg.order <= 4 && c->rows.ready) {
@@ -385,17 +386,22 @@ int viscous_buffers(dg_ctx* c) {
     }
     const bool fused = c->cfg.mu > 0.0 && c->cfg.precision == DG_PREC_FP64;
     if (c->cfg.order >= 1 && c->cfg.order <= 4 && (fused || c->nowned >= (int64_t)kVisc8PerSm * kRows8 * c->sms)) {
-        std::vector<FaceInfo> hfi(c->nface);
-        std::vector<ElemFace> hef(4 * c->ncell);
-        std::vector<double> hgeo(10 * c->ncell);
+        std::vector<FaceInfo> hfi;
+        std::vector<ElemFace> hef;
         std::vector<FaceGroup8> fg;
         std::vector<ElemGroup8> eg;
-        DG_CUDA(cudaMemcpy(hfi.data(), c->d_fi, sizeof(FaceInfo) * hfi.size(), cudaMemcpyDeviceToHost));
-        DG_CUDA(cudaMemcpy(hef.data(), c->d_ef, sizeof(ElemFace) * hef.size(), cudaMemcpyDeviceToHost));
-        if (rows8_groups(c->cfg.order, c->qv, c->qf, hfi, hef, c->nowned, fg, eg)) {
-            DG_CUDA(cudaMemcpy(hgeo.data(), c->d_geo, sizeof(double) * hgeo.size(), cudaMemcpyDeviceToHost));
+        if (!faces) {
+            hfi.resize(c->nface);
+            hef.resize(4 * c->ncell);
+            DG_CUDA(cudaMemcpy(hfi.data(), c->d_fi, sizeof(FaceInfo) * hfi.size(), cudaMemcpyDeviceToHost));
+            DG_CUDA(cudaMemcpy(hef.data(), c->d_ef, sizeof(ElemFace) * hef.size(), cudaMemcpyDeviceToHost));
+        }
+        if (rows8_groups(c->cfg.order, c->qv, c->qf, faces ? *faces : hfi, faces ? *elems : hef, c->nowned, fg, eg)) {
             c->visc8.own.sms = c->sms;
-            int rc = init_rows8(c->visc8.own, t, hgeo, fg, eg, c->ncell, c->nface, c->qv, c->qf, false);
+            c->visc8.own.maps = face_maps_of(faces ? *faces : hfi);
+            c->visc8.own.jd = c->tc.jd;  // the same numbers, if there
+            c->visc8.own.inv_detj = c->tc.inv_detj;
+            int rc = init_rows8(c->visc8.own, t, c->d_geo, fg, eg, c->ncell, c->nface, c->qv, c->qf, false);
             if (rc) return rc;
             c->visc8.rows = &c->visc8.own;
             return init_visc8(c->visc8, t, c->nface, c->qf);
@@ -801,7 +807,8 @@ dg_ctx* create_impl(const dg_mesh_desc* mesh, const dg_config* cfg, int* err, co
     }
     if (rows) {
         c->rows.sms = c->sms;
-        if ((rc = init_rows8(c->rows, c->tab, hgeo, fg8, eg8, c->ncell, c->nface, qv, qf))) return fail(c, rc);
+        c->rows.maps = face_maps_of(hfi);
+        if ((rc = init_rows8(c->rows, c->tab, c->d_geo, fg8, eg8, c->ncell, c->nface, qv, qf))) return fail(c, rc);
     } else if (cfg->precision == DG_PREC_FP64 && tc_supported(cfg->order, qv, qf)) {
         if ((rc = init_tc(c->tc, c->tab, hgeo, hfi, hef, c->ncell, c->nowned, c->nface, qv, qf))) return fail(c, rc);
     }
@@ -821,7 +828,7 @@ dg_ctx* create_impl(const dg_mesh_desc* mesh, const dg_config* cfg, int* err, co
     }
     // Navier-Stokes stepping: the viscous buffers now, so that no step allocates (graph capture)
     if (cfg->mu > 0.0) {
-        if ((rc = viscous_buffers(c)) ||
+        if ((rc = viscous_buffers(c, &hfi, &hef)) ||
             (rc = dev_alloc(&c->d_Rv, fused_navier_stokes(c) ? 0 : (size_t)c->ncell * 5 * nb)))
             return fail(c, rc);
         c->mixed.Rv = c->d_Rv;

@@ -4,6 +4,7 @@
 
 #include "dg_fp64_rows.h"
 #include "dg_mixed_host.cuh"
+#include "dg_status.cuh"
 #include "dg_viscous_rows.h"
 
 namespace fvedg {
@@ -13,6 +14,7 @@ struct Rows8Data {
     int order = 0, qv = 0, qf = 0;
     int nfgroups = 0, negroups = 0;
     int sms = 148;
+    uint32_t maps = 0;  // the face maps (bit p) that the mesh has: a box of cubes has a third of the 24
     std::vector<void*> bufs;
     Rows8Tables t{};
     const FaceGroup8* fgroups = nullptr;
@@ -68,7 +70,24 @@ inline bool rows8_groups(int order, int qv, int qf, const std::vector<FaceInfo>&
     return (int64_t)eg.size() * kRows8 * 3 <= nowned * 4 && (int64_t)fg.size() * kRows8 * 3 <= (int64_t)hfi.size() * 4;
 }
 
-inline int init_rows8(Rows8Data& m, const Tables& tab, const std::vector<double>& hgeo, const std::vector<FaceGroup8>& fg,
+// det J * J^-T and 1 / det J of the cells from their geometry ([10]: J^-T, det J).
+__global__ void rows8_geometry(const double* __restrict__ geo, int64_t ncell, double* __restrict__ jd, double* __restrict__ inv_detj) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= 10 * ncell) return;
+    const int64_t e = i / 10;
+    const int k = (int)(i - 10 * e);
+    if (k < 9) jd[9 * e + k] = geo[10 * e + 9] * geo[i];
+    else inv_detj[e] = 1.0 / geo[i];
+}
+
+inline uint32_t face_maps_of(const std::vector<FaceInfo>& hfi) {
+    uint32_t maps = 0;
+    for (const FaceInfo& f : hfi) maps |= 1u << (f.meta & 0xff) | (f.c1 >= 0 ? 1u << (f.meta >> 8 & 0xff) : 0u);
+    return maps;
+}
+
+// The tables of the face maps in m.maps. geo: the cells' geometry on the device. m.jd and m.inv_detj, if set, are the same of another set of kernels.
+inline int init_rows8(Rows8Data& m, const Tables& tab, const double* geo, const std::vector<FaceGroup8>& fg,
                       const std::vector<ElemGroup8>& eg, int64_t ncell, int64_t nface, int qv, int qf,
                       bool with_records = true) {
     const int NB = tab.nb, NQV = tab.nqv, NQF = tab.nqf, NM = face_moments(NB), MR = moment_row(NB);
@@ -77,13 +96,16 @@ inline int init_rows8(Rows8Data& m, const Tables& tab, const std::vector<double>
     m.order = tab.order; m.qv = qv; m.qf = qf;
     std::vector<double> psi, norm, T, tf, tm, tv, tw, tl;
     face_moment_basis(tab.order, qf, psi, norm);
-    face_moment_maps(tab, qf, psi, norm, T);
+    face_moment_maps(tab, qf, psi, norm, T, m.maps);
+    tf.assign((size_t)24 * NF * KT * 32, 0.0);
+    tw.reserve((size_t)NV * 6 * NJ * 32);
+    tl.assign((size_t)24 * KF * NJ * 32, 0.0);
     for (int p = 0; p < 24; ++p)
-        for (int nt = 0; nt < NF; ++nt)
+        for (int nt = 0; nt < NF && (m.maps >> p & 1u); ++nt)
             for (int kt = 0; kt < KT; ++kt)
                 for (int l = 0; l < 32; ++l) {
                     const int g = 8 * nt + l / 4, b = 4 * kt + l % 4;
-                    tf.push_back(g < NQF && b < NB ? tab.phi_f[((size_t)p * NQF + g) * NB + b] : 0.0);
+                    if (g < NQF && b < NB) tf[((size_t)(p * NF + nt) * KT + kt) * 32 + l] = tab.phi_f[((size_t)p * NQF + g) * NB + b];
                 }
     for (int nt = 0; nt < NF; ++nt)
         for (int i = 0; i < 2; ++i)
@@ -107,7 +129,7 @@ inline int init_rows8(Rows8Data& m, const Tables& tab, const std::vector<double>
                         tw.push_back(g < NQV && b < NB ? tab.dphi_vw[((size_t)g * NB + b) * 3 + d] : 0.0);
                     }
     std::vector<double> mv;
-    for (int j = 0; j < NJ; ++j)
+    for (int j = 0; j < NJ && short_sums8(NB); ++j)
         for (int l = 0; l < 32; ++l) {
             const int b = 8 * j + l / 4, d = l % 4;
             long double s = 0;
@@ -116,28 +138,32 @@ inline int init_rows8(Rows8Data& m, const Tables& tab, const std::vector<double>
             mv.push_back((double)s);
         }
     for (int p = 0; p < 24; ++p)
-        for (int t = 0; t < KF; ++t)
+        for (int t = 0; t < KF && (m.maps >> p & 1u); ++t)
             for (int j = 0; j < NJ; ++j)
                 for (int l = 0; l < 32; ++l) {
                     const int k = moment_of(NB, t, l % 4), b = 8 * j + l / 4;
-                    tl.push_back(k < NM && b < NB ? T[((size_t)p * NB + b) * NM + k] : 0.0);
+                    if (k < NM && b < NB) tl[((size_t)(p * KF + t) * NJ + j) * 32 + l] = T[((size_t)p * NB + b) * NM + k];
                 }
-    std::vector<double> inv_mass(NB), jd(9 * ncell), inv_detj(ncell);
+    std::vector<double> inv_mass(NB);
     for (int j = 0; j < NB; ++j) inv_mass[j] = 1.0 / tab.mass_ref[j];
-    for (int64_t e = 0; e < ncell; ++e) {
-        const double dj = hgeo[10 * e + 9];
-        for (int i = 0; i < 9; ++i) jd[9 * e + i] = dj * hgeo[10 * e + i];
-        inv_detj[e] = 1.0 / dj;
-    }
     m.nfgroups = (int)fg.size();
     m.negroups = (int)eg.size();
     int rc;
     if ((rc = rows8_upload(m, &m.t.tf, tf)) || (rc = rows8_upload(m, &m.t.tm, tm)) || (rc = rows8_upload(m, &m.t.tv, tv)) ||
         (rc = rows8_upload(m, &m.t.tw, tw)) || (rc = rows8_upload(m, &m.t.tl, tl)) ||
-        (rc = rows8_upload(m, &m.t.mv, mv)) || (rc = rows8_upload(m, &m.t.inv_mass, inv_mass)) || (rc = rows8_upload(m, &m.jd, jd)) ||
-        (rc = rows8_upload(m, &m.inv_detj, inv_detj)) || (rc = rows8_upload(m, &m.fgroups, fg)) ||
+        (rc = rows8_upload(m, &m.t.mv, mv)) || (rc = rows8_upload(m, &m.t.inv_mass, inv_mass)) || (rc = rows8_upload(m, &m.fgroups, fg)) ||
         (rc = rows8_upload(m, &m.egroups, eg)))
         return rc;
+    if (!m.jd) {
+        void* p = nullptr;
+        if (cudaMalloc(&p, sizeof(double) * 10 * ncell) != cudaSuccess) return DG_E_NOMEM;
+        m.bufs.push_back(p);
+        double* jd = (double*)p;
+        rows8_geometry<<<(unsigned)((10 * ncell + 255) / 256), 256>>>(geo, ncell, jd, jd + 9 * ncell);
+        if ((rc = cuda_status(cudaGetLastError())) || (rc = cuda_status(cudaStreamSynchronize(0)))) return rc;
+        m.jd = jd;
+        m.inv_detj = jd + 9 * ncell;
+    }
     if (with_records) {
         void* p = nullptr;
         const size_t n = sizeof(double) * nface * 5 * MR;
@@ -172,14 +198,18 @@ inline int init_visc8(Visc8Data& m, const Tables& tab, int64_t nface, int qf) {
     const int KT = (NB + 3) / 4, NF = pad8(NQF) / 8, NV = pad8(NQV) / 8, NJ = pad8(NB) / 8, KD = deriv_ktiles(NB);
     std::vector<double> psi, norm, tfd, tvd, td;
     face_moment_basis(tab.order, qf, psi, norm);
-    const double* r = tri_rule(qf);
+    const uint32_t maps = m.rows->maps;
+    tfd.assign((size_t)24 * NF * KT * 96, 0.0);
+    tvd.reserve((size_t)NV * KT * 96);
+    td.assign((size_t)72 * KD * NJ * 32, 0.0);
     for (int p = 0; p < 24; ++p)
-        for (int nt = 0; nt < NF; ++nt)
+        for (int nt = 0; nt < NF && (maps >> p & 1u); ++nt)
             for (int kt = 0; kt < KT; ++kt)
                 for (int d = 0; d < 3; ++d)
                     for (int l = 0; l < 32; ++l) {
                         const int g = 8 * nt + l / 4, b = 4 * kt + l % 4;
-                        tfd.push_back(g < NQF && b < NB ? tab.dphi_f[(((size_t)p * NQF + g) * NB + b) * 3 + d] : 0.0);
+                        if (g < NQF && b < NB)
+                            tfd[((size_t)((p * NF + nt) * KT + kt) * 3 + d) * 32 + l] = tab.dphi_f[(((size_t)p * NQF + g) * NB + b) * 3 + d];
                     }
     for (int nt = 0; nt < NV; ++nt)
         for (int kt = 0; kt < KT; ++kt)
@@ -188,20 +218,36 @@ inline int init_visc8(Visc8Data& m, const Tables& tab, int64_t nface, int qf) {
                     const int g = 8 * nt + l / 4, b = 4 * kt + l % 4;
                     tvd.push_back(g < NQV && b < NB ? tab.dphi_v[((size_t)g * NB + b) * 3 + d] : 0.0);
                 }
-    // D[perm][d][j][m] = sum_g w_g dphi_j,d psi_m / |psi_m|^2; degree P - 1, so moments past that vanish
-    const int nd = tab.order * (tab.order + 1) / 2;
-    for (int p = 0; p < 24; ++p)
+    // D[perm][d][j][m] = sum_g w_g dphi_j,d psi_m / |psi_m|^2; zero for moments past the derivative's degree
+    const std::vector<long double> w = moment_projection(qf, psi, norm);
+    std::vector<double> D((size_t)3 * NB * NM), dphi((size_t)3 * NB * NQF);
+    for (int p = 0; p < 24; ++p) {
+        if (!(maps >> p & 1u)) continue;
+        for (int g = 0; g < NQF; ++g)
+            for (int i = 0; i < 3 * NB; ++i) dphi[(size_t)i * NQF + g] = tab.dphi_f[((size_t)p * NQF + g) * NB * 3 + i];
+        for (int b = 0; b < NB; ++b) {
+            const int deg = mode_degree(b), most = std::min(NM, deg * (deg + 1) / 2);
+            for (int d = 0; d < 3; ++d)
+                for (int k = 0; k < most; ++k) {
+                    const double* x = &dphi[(size_t)(3 * b + d) * NQF];
+                    long double s = 0, s2 = 0;
+                    int g = 0;
+                    for (; g + 1 < NQF; g += 2) {
+                        s += w[(size_t)k * NQF + g] * x[g];
+                        s2 += w[(size_t)k * NQF + g + 1] * x[g + 1];
+                    }
+                    if (g < NQF) s += w[(size_t)k * NQF + g] * x[g];
+                    D[((size_t)d * NB + b) * NM + k] = (double)(s + s2);
+                }
+        }
         for (int d = 0; d < 3; ++d)
             for (int t = 0; t < KD; ++t)
                 for (int j = 0; j < NJ; ++j)
                     for (int l = 0; l < 32; ++l) {
                         const int k = 8 * (t / 2) + 2 * (l % 4) + t % 2, b = 8 * j + l / 4;
-                        long double s = 0;
-                        if (k < std::min(nd, NM) && b < NB)
-                            for (int g = 0; g < NQF; ++g)
-                                s += (long double)r[3 * g + 2] * tab.dphi_f[(((size_t)p * NQF + g) * NB + b) * 3 + d] * psi[(size_t)k * NQF + g];
-                        td.push_back(k < std::min(nd, NM) && b < NB ? (double)(s / norm[k]) : 0.0);
+                        if (k < NM && b < NB) td[((size_t)((p * 3 + d) * KD + t) * NJ + j) * 32 + l] = D[((size_t)d * NB + b) * NM + k];
                     }
+    }
     auto up = [&](const double** dst, const std::vector<double>& v) {
         void* p = nullptr;
         if (cudaMalloc(&p, sizeof(double) * v.size()) != cudaSuccess) return (int)DG_E_NOMEM;

@@ -3,6 +3,7 @@
 #include <cmath>
 #include <cstdlib>
 
+#include "dg_groups.h"
 #include "dg_kernels_mixed.cuh"
 #include "dg_mixed16.h"
 #include "dg_mixed_combos.h"
@@ -110,63 +111,6 @@ inline void append_frag_table(const std::vector<double>& T, int N, int K, std::v
     }
 }
 
-// Faces with equal (perm0, perm1, kind) and elements with equal face maps (in canonical face
-// order: local face q is the one opposite local vertex q) are grouped in threes, in mesh order.
-// A partial group repeats its first member in the unused slots (never read as a row: rows of
-// unused slots are masked by the group size).
-// Face groups: faces of the same kind in threes, first the faces between owned elements, then
-// (from *nf_inner on) the faces touching a ghost element (cells >= ncell), whose fluxes need the
-// ghost rows of a halo exchange. Element groups: the owned elements [0, ncell).
-template <class FG, class EG>
-inline void build_groups(const std::vector<FaceInfo>& hfi, const std::vector<ElemFace>& hef, int64_t ncell,
-                         std::vector<FG>& fg, std::vector<EG>& eg, int* nf_inner) {
-    constexpr int N = sizeof(FG{}.f) / sizeof(int);
-    for (int halo = 0; halo < 2; ++halo) {
-        std::map<int64_t, FG> open_f;
-        for (int64_t f = 0; f < (int64_t)hfi.size(); ++f) {
-            const FaceInfo& F = hfi[f];
-            if ((F.c0 >= ncell || F.c1 >= ncell) != (halo == 1)) continue;
-            const int64_t key = (int64_t)(F.meta & 0xffffff) * 2 + (F.c1 >= 0 ? 1 : 0);
-            FG& g = open_f[key];
-            g.f[g.n++] = (int)f;
-            if (g.n == N) { fg.push_back(g); g = FG{}; }
-        }
-        for (auto& kv : open_f)
-            if (kv.second.n > 0) {
-                for (int i = kv.second.n; i < N; ++i) kv.second.f[i] = kv.second.f[0];
-                fg.push_back(kv.second);
-            }
-        if (halo == 0) *nf_inner = (int)fg.size();
-    }
-    std::map<int64_t, EG> open_e;  // by the four face maps and sides
-    for (int64_t e = 0; e < ncell; ++e) {
-        int face[4] = {-1, -1, -1, -1}, meta[4] = {0, 0, 0, 0};
-        for (int i = 0; i < 4; ++i) {
-            const ElemFace& ef = hef[4 * e + i];
-            const int p = ef.meta & 0xff;
-            const int q = 6 - kPermSlots[p][0] - kPermSlots[p][1] - kPermSlots[p][2];  // missing vertex
-            face[q] = ef.face;
-            meta[q] = ef.meta;
-        }
-        int64_t key = 0;
-        for (int q = 0; q < 4; ++q) key = key * 65536 + meta[q];
-        EG& g = open_e[key];
-        g.e[g.n] = (int)e;
-        for (int q = 0; q < 4; ++q) { g.face[g.n][q] = face[q]; g.meta[q] = meta[q]; }
-        ++g.n;
-        if (g.n == N) { eg.push_back(g); g = EG{}; }
-    }
-    for (auto& kv : open_e)
-        if (kv.second.n > 0) {
-            EG g = kv.second;
-            for (int i = g.n; i < N; ++i) {
-                g.e[i] = g.e[0];
-                for (int q = 0; q < 4; ++q) g.face[i][q] = g.face[0][q];
-            }
-            eg.push_back(g);
-        }
-}
-
 // A basis of the polynomials of degree <= order on the triangle, orthogonal under the face rule, with
 // psi_0 = 1: monomials u^i v^j by degree, Gram-Schmidt (twice) in the rule's inner product, whose
 // exactness makes it a true one up to that degree. psi[m][g], norm[m] = sum_g w_g psi_m^2.
@@ -198,21 +142,49 @@ inline void face_moment_basis(int order, int qf, std::vector<double>& psi, std::
     norm.assign(nn.begin(), nn.end());
 }
 
-// T[perm][j][m] with phi_j(xi^perm_g) = sum_m T psi_m(g) at every face point.
-inline void face_moment_maps(const Tables& tab, int qf, const std::vector<double>& psi, const std::vector<double>& norm,
-                             std::vector<double>& T) {
-    const int nb = tab.nb, nq = tab.nqf, nm = (int)norm.size();
+// Total degree of mode j of the basis on the tetrahedron, which is listed by degree (as the moments are).
+inline int mode_degree(int j) {
+    int d = 0;
+    while (j >= (d + 1) * (d + 2) * (d + 3) / 6) ++d;
+    return d;
+}
+
+// The projection onto the moments, w_g psi_m(g) / |psi_m|^2, [m][g].
+inline std::vector<long double> moment_projection(int qf, const std::vector<double>& psi, const std::vector<double>& norm) {
+    const int nq = tri_rule_npts(qf);
     const double* r = tri_rule(qf);
+    std::vector<long double> w(psi.size());
+    for (size_t m = 0; m < norm.size(); ++m)
+        for (int g = 0; g < nq; ++g) w[m * nq + g] = (long double)r[3 * g + 2] * psi[m * nq + g] / norm[m];
+    return w;
+}
+
+// T[perm][j][m] with phi_j(xi^perm_g) = sum_m T psi_m(g) at every face point; zero for moments of a higher degree
+// than the mode's, and for face maps that are not in `maps`.
+inline void face_moment_maps(const Tables& tab, int qf, const std::vector<double>& psi, const std::vector<double>& norm,
+                             std::vector<double>& T, uint32_t maps = 0xffffffu) {
+    const int nb = tab.nb, nq = tab.nqf, nm = (int)norm.size();
+    const std::vector<long double> w = moment_projection(qf, psi, norm);
     T.assign((size_t)24 * nb * nm, 0.0);
-    for (int p = 0; p < 24; ++p)
-        for (int j = 0; j < nb; ++j)
-            for (int m = 0; m < nm; ++m) {
-                if (j == 0) { T[((size_t)p * nb) * nm + m] = m == 0 ? 1.0 : 0.0; continue; }  // phi_0 = psi_0 = 1
-                long double s = 0;
-                for (int g = 0; g < nq; ++g)
-                    s += (long double)r[3 * g + 2] * tab.phi_f[((size_t)p * nq + g) * nb + j] * psi[(size_t)m * nq + g];
-                T[((size_t)p * nb + j) * nm + m] = (double)(s / norm[m]);
+    for (int p = 0; p < 24; ++p) {
+        if (!(maps >> p & 1u)) continue;
+        T[(size_t)p * nb * nm] = 1.0;  // phi_0 = psi_0 = 1
+        for (int j = 1; j < nb; ++j) {
+            const int d = mode_degree(j), most = std::min(nm, (d + 1) * (d + 2) / 2);
+            const double* phi = &tab.phi_fT[((size_t)p * nb + j) * nq];
+            for (int m = 0; m < most; ++m) {
+                const long double* wm = &w[(size_t)m * nq];
+                long double s = 0, s2 = 0;  // two chains, for the speed
+                int g = 0;
+                for (; g + 1 < nq; g += 2) {
+                    s += wm[g] * phi[g];
+                    s2 += wm[g + 1] * phi[g + 1];
+                }
+                if (g < nq) s += wm[g] * phi[g];
+                T[((size_t)p * nb + j) * nm + m] = (double)(s + s2);
             }
+        }
+    }
 }
 
 // Tables, groups and records of the kernels for groups of sixteen.
