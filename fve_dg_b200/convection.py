@@ -116,7 +116,7 @@ class ExplicitConvection:
         return json.loads(buf.value.decode())
 
     def set_element_shape(self, staged, ctas_per_sm=1):
-        """Pin the two-launch element kernel's shape (a choice dg_autotune records)."""
+        """Pin the two-launch element kernel's shape (a choice dg_autotune records); no effect in groups of sixteen."""
         L.check(L.lib().dg_set_element_shape(self._ctx, int(bool(staged)), int(ctas_per_sm)), "dg_set_element_shape")
 
     def kernel_group(self, viscous=False):

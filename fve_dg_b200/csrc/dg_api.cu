@@ -1394,6 +1394,7 @@ int dg_autotune(dg_ctx* c, double dt, char* report, size_t len) {
     cudaEventCreate(&e1);
     std::string js = "{\"order\": " + std::to_string(c->cfg.order) + ", \"quad_vol\": " + std::to_string(c->qv) +
                      ", \"quad_face\": " + std::to_string(c->qf) + ", \"ncell\": " + std::to_string(c->ncell) +
+                     ", \"items_per_group\": " + std::to_string(c->qs.group) +
                      ", \"face_groups\": " + std::to_string(c->mixed.nfgroups) +
                      ", \"element_groups\": " + std::to_string(c->mixed.negroups) + ", \"candidates\": [";
     float best = 1e30f;
@@ -1415,8 +1416,8 @@ int dg_autotune(dg_ctx* c, double dt, char* report, size_t len) {
         float ms = 0.f;
         cudaEventElapsedTime(&ms, e0, e1);
         ms *= 0.5f;
-        js += std::string(i ? ", " : "") + "{\"tile_f\": " + std::to_string(cand[i][0]) + ", \"tile_e\": " +
-              std::to_string(cand[i][1]) + ", \"max_blocks_per_sm\": " + std::to_string(cand[i][2]) +
+        js += std::string(i ? ", " : "") + "{\"tile_f\": " + std::to_string(c->qs.tile_f) + ", \"tile_e\": " +
+              std::to_string(c->qs.tile_e) + ", \"max_blocks_per_sm\": " + std::to_string(cand[i][2]) +
               ", \"regions\": " + std::to_string(c->qs.nregions) + ", \"lag\": " + std::to_string(cand[i][4]) +
               ", \"ms_per_step\": " + std::to_string(ms) + "}";
         if (rc == DG_OK && ms < best) { best = ms; bestp = c->pp; }
@@ -1426,8 +1427,8 @@ int dg_autotune(dg_ctx* c, double dt, char* report, size_t len) {
         const int brc = build_schedule(c->mixed, c->qs, c->pp);
         if (rc == DG_OK) rc = brc;
     }
-    js += "], \"chosen\": {\"tile_f\": " + std::to_string(bestp.tile_f) + ", \"tile_e\": " +
-          std::to_string(bestp.tile_e) + ", \"max_blocks_per_sm\": " + std::to_string(bestp.max_blocks) +
+    js += "], \"chosen\": {\"tile_f\": " + std::to_string(c->qs.tile_f) + ", \"tile_e\": " +
+          std::to_string(c->qs.tile_e) + ", \"max_blocks_per_sm\": " + std::to_string(bestp.max_blocks) +
           ", \"regions\": " + std::to_string(c->qs.nregions) + ", \"lag\": " + std::to_string(bestp.lag) +
           ", \"ms_per_step\": " + std::to_string(best) + "}}";
     cudaMemcpyAsync(c->d_Un, save, nstate * sizeof(double), cudaMemcpyDeviceToDevice, c->stream);

@@ -87,9 +87,7 @@ int run_element(int sms, const Mixed16ElemArgs& a, cudaStream_t s) {
 }
 
 template <int NB, int NQV, int NQF>
-int run_stage(int sms, const Mixed16FaceArgs& fa, const Mixed16ElemArgs& ea, const TileQueue& q, int max_blocks,
-              cudaStream_t s) {
-    (void)max_blocks;  // one CTA per SM in any case
+int run_stage(int sms, const Mixed16FaceArgs& fa, const Mixed16ElemArgs& ea, const TileQueue& q, cudaStream_t s) {
     constexpr size_t tables = ElemSizes16<NB, NQV>::tables, warp = stage_warp_smem<NB, NQV, NQF>();
     constexpr int W = warps16(NB <= 10 ? 12 : 8, warp, tables);
     constexpr size_t smem = tables + warp * W;
@@ -118,9 +116,9 @@ int mixed16_element(int order, int qv, int qf, int sms, const Mixed16ElemArgs& a
 }
 
 int mixed16_stage(int order, int qv, int qf, int sms, const Mixed16FaceArgs& fa, const Mixed16ElemArgs& ea,
-                  const TileQueue& q, int max_blocks, cudaStream_t s) {
+                  const TileQueue& q, cudaStream_t s) {
 #define X(P, QV, QF, NB, NQV, NQF, W) \
-    if (order == P && qv == QV && qf == QF) return run_stage<NB, NQV, NQF>(sms, fa, ea, q, max_blocks, s);
+    if (order == P && qv == QV && qf == QF) return run_stage<NB, NQV, NQF>(sms, fa, ea, q, s);
     FVEDG_MIXED_COMBOS(X)
 #undef X
     return DG_E_ARG;

@@ -12,7 +12,7 @@ int mixed16_face(int order, int qv, int qf, int sms, const Mixed16FaceArgs& a, c
 int mixed16_element(int order, int qv, int qf, int sms, const Mixed16ElemArgs& a, cudaStream_t s);
 // One stage as a persistent launch over the tile list.
 int mixed16_stage(int order, int qv, int qf, int sms, const Mixed16FaceArgs& fa, const Mixed16ElemArgs& ea,
-                  const TileQueue& q, int max_blocks, cudaStream_t s);
+                  const TileQueue& q, cudaStream_t s);
 // Warps of the element kernel's CTA (one per SM).
 int mixed16_element_warps(int order, int qv, int qf);
 

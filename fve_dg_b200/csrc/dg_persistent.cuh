@@ -25,7 +25,7 @@ namespace fvedg {
 constexpr long long kSpinLimit = 1ll << 24;  // about a second of 64 ns naps
 
 struct PersistentParams {
-    int tile_f = 32;     // face groups per tile
+    int tile_f = 32;     // face groups per tile, in groups of three (build_schedule has those of sixteen)
     int tile_e = 16;     // element groups per tile
     int max_blocks = 0;  // CTAs per SM cap (0 = as many as fit)
     int regions = 32;    // element regions (1 .. kMaxRegions)
@@ -41,6 +41,7 @@ struct QueueSchedule {
     unsigned long long* deps = nullptr; // [R] face regions each element region reads
     unsigned int* total = nullptr;      // [R] face groups per region
     int ntiles = 0, nregions = 0;
+    int group = 0, tile_f = 0, tile_e = 0;  // items per group, and the groups per tile of the list
     PersistentParams built{};
     bool ready = false;
 };
@@ -94,6 +95,9 @@ inline int build_schedule_of(MixedData& m, std::vector<FG>& hfg, const std::vect
     if (ne < 1 || nf < 1) return DG_E_ARG;
     const int R = std::max(1, std::min({pp.regions, kMaxRegions, ne}));
     const int tf = std::max(1, tile_f), te = std::max(1, tile_e), lag = std::max(0, pp.lag);
+    qs.group = (int)(sizeof(FG{}.f) / sizeof(int));
+    qs.tile_f = tf;
+    qs.tile_e = te;
     std::vector<int> ereg(m.ncell, R), greg(ne);  // ghost cells (in no element group) stay at R
     for (int g = 0; g < ne; ++g) {
         greg[g] = (int)((int64_t)g * R / ne);
@@ -173,7 +177,8 @@ inline int build_schedule_of(MixedData& m, std::vector<FG>& hfg, const std::vect
 }
 
 // Tiles are given in groups of three; a context of groups of sixteen takes about as many items per face tile
-// and as many groups per element tile as per face tile, so that the CTA's warps have one or more each.
+// and as many groups per element tile as per face tile, so that the CTA's warps have one or more each (tile_e is not
+// used there, nor max_blocks: its kernel has one CTA per SM).
 inline int build_schedule(MixedData& m, QueueSchedule& qs, const PersistentParams& pp) {
     if (m.wide) {
         const int t = std::max(3, pp.tile_f * 3 / 8);
@@ -227,8 +232,7 @@ inline int persistent_kernel(MixedData& m, QueueState* q, const QueueSchedule& q
     if (m.wide) {
         if (!qs.ready || !(qs.built == pp)) return DG_E_STATE;
         return mixed16_stage(m.order, m.qv, m.qf, m.sms, face_args16(m, U, face_mask),
-                             elem_args16(m, U, U0, out, mode, dt, a0, a1, with_volume), tile_queue(q, qs, pp),
-                             pp.max_blocks, s);
+                             elem_args16(m, U, U0, out, mode, dt, a0, a1, with_volume), tile_queue(q, qs, pp), s);
     }
 #define X(P, QV, QF, NB, NQV, NQF, W)                                                                              \
     if (m.order == P && m.qv == QV && m.qf == QF)                                                                  \

@@ -172,3 +172,31 @@ def test_viscous_operator_between_the_convective_lines(precision):
         assert c.kernel_group() == 3 and c.kernel_group(viscous=True) == 8
         c.close()
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("P,n,group", [(2, 17, 16), (2, 8, 3)])
+def test_autotune_reports_the_tiles_that_ran(P, n, group):
+    m = box_mesh(n, jitter=0.1, seed=5)
+    c = ExplicitConvection(m, order=P, quad_vol=1, quad_face=2, precision="mixed", schedule="persistent")
+    assert c.kernel_group() == group
+    U = state(m, P)
+    c.set_state(U)
+    rec = c.autotune(1e-4)
+    tiles = {(x["tile_f"], x["tile_e"]) for x in rec["candidates"]}
+    # asked for in groups of three; groups of sixteen: three eighths as many, of faces and elements alike
+    asked = {(32, 16), (16, 8), (64, 32), (128, 64)}
+    assert rec["items_per_group"] == group
+    assert tiles == (asked if group == 3 else {(f * 3 // 8, f * 3 // 8) for f, _ in asked})
+    assert (rec["chosen"]["tile_f"], rec["chosen"]["tile_e"]) in tiles
+    assert np.array_equal(c.get_state(), U)
+    c.close()
+    # the shape of the two-launch element kernel: one in groups of sixteen, pinned or not
+    c = ExplicitConvection(m, order=P, quad_vol=1, quad_face=2, precision="mixed")
+    assert len(c.set_state(U) or c.autotune(1e-4)["candidates"]) == (1 if group == 16 else 3)
+    out = []
+    for staged in (False, True):
+        c.set_element_shape(staged, 1)
+        c.set_state(U)
+        c.ssprk3(1e-4, 1)
+        out.append(c.get_state())
+    assert np.array_equal(out[0], out[1])
