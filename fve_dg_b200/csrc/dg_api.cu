@@ -306,7 +306,6 @@ Rows8ElemArgs rows8_elem_args(dg_ctx* c, const double* U, const double* U0, doub
     a.groups = c->rows.egroups; a.ngroups = c->rows.negroups; a.t = c->rows.t; a.gamma = c->cfg.gamma;
     a.with_volume = with_volume; a.mode = mode; a.dt = dt; a.a0 = a0; a.a1 = a1;
     a.dt_inst = mode == 1 ? c->d_dt_inst : nullptr; a.elem_inst = c->d_elem_inst;
-    a.Rv = (mode == 1 && c->cfg.mu > 0.0) ? c->d_Rv : nullptr;
     a.err = c->rows.err;
     return a;
 }
@@ -453,7 +452,7 @@ Visc8Args visc8_args(dg_ctx* c, const double* U, const double* U0, double* out, 
     v.e.U = U; v.e.U0 = U0; v.e.out = out; v.e.rec = c->visc8.rec; v.e.jd = r.jd; v.e.inv_detj = r.inv_detj;
     v.e.groups = r.egroups; v.e.ngroups = r.negroups; v.e.t = r.t; v.e.gamma = c->cfg.gamma; v.e.with_volume = 1;
     v.e.mode = mode; v.e.dt = dt; v.e.a0 = a0; v.e.a1 = a1;
-    v.e.dt_inst = mode == 1 ? c->d_dt_inst : nullptr; v.e.elem_inst = c->d_elem_inst; v.e.Rv = nullptr; v.e.err = r.err;
+    v.e.dt_inst = mode == 1 ? c->d_dt_inst : nullptr; v.e.elem_inst = c->d_elem_inst; v.e.err = r.err;
     v.v = c->visc8.v; v.geo = c->d_geo; v.h = c->d_h; v.mu = mu; v.cq = c->cfg.gamma / prandtl; v.order = c->cfg.order;
     return v;
 }

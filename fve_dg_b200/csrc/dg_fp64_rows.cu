@@ -8,17 +8,6 @@
 namespace fvedg {
 namespace {
 
-template <class Kernel>
-int opt_in(Kernel k, size_t smem, unsigned long long& done_mask) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return DG_E_CUDA;
-    const unsigned long long bit = 1ull << (dev & 63);
-    if (done_mask & bit) return DG_OK;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return DG_E_CUDA;
-    done_mask |= bit;
-    return DG_OK;
-}
-
 // Resident warps per SM, by the registers a thread needs: sixteen at 128 up to P2 (P1 face kernel 0.090 against
 // 0.104 ms with twelve, element kernel 0.077 against 0.090, 196,608 tets), twelve at 168 at P3 (face 0.352 against
 // 0.391 ms with eight), eight at 255 above.
@@ -29,7 +18,7 @@ int run_face(int sms, const Rows8FaceArgs& a, cudaStream_t s) {
     constexpr int W = warps16(most_warps(NB), sizeof(FaceSmem8<NB>));
     constexpr size_t smem = sizeof(FaceSmem8<NB>) * W;
     static unsigned long long done = 0;
-    if (const int rc = opt_in(face_flux_rows8<NB, NQF, W>, smem, done)) return rc;
+    if (const int rc = ensure_smem(face_flux_rows8<NB, NQF, W>, smem, done)) return rc;
     return a.ngroups > 0 ? launch_early(face_flux_rows8<NB, NQF, W>, std::min(a.ngroups, sms), W * 32, smem, s, a) : (int)DG_OK;
 }
 
@@ -38,7 +27,7 @@ int run_element(int sms, const Rows8ElemArgs& a, cudaStream_t s) {
     constexpr int W = warps16(most_warps(NB), sizeof(ElemSmem8<NB>));
     constexpr size_t smem = sizeof(ElemSmem8<NB>) * W;
     static unsigned long long done = 0;
-    if (const int rc = opt_in(element_rows8<NB, NQV, W>, smem, done)) return rc;
+    if (const int rc = ensure_smem(element_rows8<NB, NQV, W>, smem, done)) return rc;
     return a.ngroups > 0 ? launch_early(element_rows8<NB, NQV, W>, std::min(a.ngroups, sms), W * 32, smem, s, a) : (int)DG_OK;
 }
 

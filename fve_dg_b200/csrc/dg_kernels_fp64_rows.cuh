@@ -86,10 +86,9 @@ struct Rows8ElemArgs {
     double gamma;
     int with_volume;
     int mode;
-    double dt, a0, a1;       // out = a0 U0 + a1 (U + dt (-(R - Rv) / b))
+    double dt, a0, a1;       // out = a0 U0 + a1 (U - dt R / b)
     const double* dt_inst;
     const int* elem_inst;
-    const double* Rv;
     int* err;
 };
 
@@ -380,7 +379,7 @@ __device__ __forceinline__ bool element_group8(const Rows8ElemArgs& a, int gi, E
     #pragma unroll 1
     for (int q = 0; q < 4; ++q) {
         const int meta = grp.meta[q];
-        const double sgn = (meta >> 8) ? -1.0 : 1.0;
+        const double sgn = (meta >> 8) ? -1.0 : 1.0, smom = SHORT ? 1.0 : sgn;  // on the moments, or on the face's sum
         const double* rec = a.rec + (int64_t)grp.face[gid][q] * (5 * MR);
         const double* tb = a.t.tl + (int64_t)(meta & 0xff) * KF * NJ * 32 + lane;
         double m[5][KF];
@@ -392,12 +391,12 @@ __device__ __forceinline__ bool element_group8(const Rows8ElemArgs& a, int gi, E
                 for (int k = 0; k < 5; ++k) {
                     double2 x = make_double2(0.0, 0.0);
                     if (8 * (t / 2) + 8 <= MR || m0 < MR) x = __ldcg(reinterpret_cast<const double2*>(rec + k * MR + m0));
-                    m[k][t] = sgn * x.x;
-                    m[k][t + 1] = sgn * x.y;
+                    m[k][t] = smom * x.x;
+                    m[k][t + 1] = smom * x.y;
                 }
             } else {
                 #pragma unroll
-                for (int k = 0; k < 5; ++k) m[k][t] = m0 < MR ? sgn * __ldcg(rec + k * MR + m0) : 0.0;
+                for (int k = 0; k < 5; ++k) m[k][t] = m0 < MR ? smom * __ldcg(rec + k * MR + m0) : 0.0;
             }
         }
         if constexpr (SHORT) {
@@ -411,7 +410,10 @@ __device__ __forceinline__ bool element_group8(const Rows8ElemArgs& a, int gi, E
                     for (int k = 0; k < 5; ++k) dmma884(part[k], m[k][t], b);
                 }
                 #pragma unroll
-                for (int k = 0; k < 5; ++k) { acc[k][j][0] += part[k][0]; acc[k][j][1] += part[k][1]; }
+                for (int k = 0; k < 5; ++k) {
+                    acc[k][j][0] = fma(sgn, part[k][0], acc[k][j][0]);
+                    acc[k][j][1] = fma(sgn, part[k][1], acc[k][j][1]);
+                }
             }
         } else {
             #pragma unroll
@@ -442,9 +444,7 @@ __device__ __forceinline__ bool element_group8(const Rows8ElemArgs& a, int gi, E
                 const double s = sdt * __ldg(a.t.inv_mass + b);
                 #pragma unroll
                 for (int k = 0; k < 5; ++k) {
-                    double R = acc[k][j][i];
-                    if (a.Rv) R -= a.Rv[e * B5 + 5 * b + k];
-                    const double x = row[5 * b + k] - s * R;
+                    const double x = row[5 * b + k] - s * acc[k][j][i];
                     os[5 * b + k] = u0 ? fma(a.a1, x, a.a0 * row0[5 * b + k]) : a.a1 * x;
                 }
             }

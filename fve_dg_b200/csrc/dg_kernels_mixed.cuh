@@ -220,13 +220,11 @@ __device__ __forceinline__ void load_afrag(AFrag<K>& A, const uint32_t* r0, cons
 // Rows gid and gid + 8 of an A operand straight from FP64 state rows (null: a zero row): r points
 // at a cell's variable-k coefficients, mode b at r[5 b]; column x of the row is mode x + 1 (the
 // deviation modes), split into BF16 hi/lo in registers exactly as a stored split row would be.
-template <int K, int NB, bool SMEM = false>
+template <int K, int NB>
 __device__ __forceinline__ void load_afrag_state(AFrag<K>& A, const double* r0, const double* r1, int lane) {
     const int tq = lane & 3;
     auto v = [&](const double* r, int x) -> float {
-        if (!r || x + 1 >= NB) return 0.f;
-        if constexpr (SMEM) return (float)r[5 * (x + 1)];
-        else return (float)r[5 * (x + 1)];
+        return !r || x + 1 >= NB ? 0.f : (float)r[5 * (x + 1)];
     };
     #pragma unroll
     for (int t = 0; t < KTiles<K>::N16; ++t) {
@@ -862,7 +860,7 @@ __device__ __forceinline__ bool element_group_staged(const MixedElemArgs& a, int
     if (a.volume) {
         {   // values at the volume points
             AFrag<KB> A;
-            load_afrag_state<KB, NB, true>(A, v0 ? st.U[r0 / 5] + r0 % 5 : nullptr,
+            load_afrag_state<KB, NB>(A, v0 ? st.U[r0 / 5] + r0 % 5 : nullptr,
                                            v1 ? st.U[r1 / 5] + r1 % 5 : nullptr, lane);
             const float c00 = sm.sC0[r0], c01 = sm.sC0[r1];
             #pragma unroll

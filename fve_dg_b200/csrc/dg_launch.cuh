@@ -33,6 +33,19 @@ __device__ __forceinline__ double ld_earlier(const double* p) {
     return v;
 }
 
+// Opt a kernel into `smem` bytes of dynamic shared memory once per device.
+template <class Kernel>
+inline int ensure_smem(Kernel k, size_t smem, unsigned long long& done_mask) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return DG_E_CUDA;
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (done_mask & bit) return DG_OK;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return DG_E_CUDA;
+    done_mask |= bit;
+    return DG_OK;
+}
+
 // Only for kernels that call await_previous() in every warp.
 template <class... P, class... A>
 inline int launch_early(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, const A&... args) {

@@ -49,17 +49,6 @@ __global__ void __launch_bounds__(WARPS * 32, 1) stage_persistent_mixed16(Mixed1
     if (threadIdx.x == 0) leave_queue(Q);
 }
 
-template <class Kernel>
-int opt_in(Kernel k, size_t smem, unsigned long long& done_mask) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return DG_E_CUDA;
-    const unsigned long long bit = 1ull << (dev & 63);
-    if (done_mask & bit) return DG_OK;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return DG_E_CUDA;
-    done_mask |= bit;
-    return DG_OK;
-}
-
 // Resident warps per SM: twelve at 168 registers a thread where that is enough, else eight at 255.
 template <int NB, int NQF>
 constexpr int face_warps() { return warps16(NB <= 20 ? 12 : 8, sizeof(FaceSmem16<NB, NQF>)); }
@@ -73,7 +62,7 @@ int run_face(int sms, const Mixed16FaceArgs& a, cudaStream_t s) {
     constexpr int W = face_warps<NB, NQF>();
     constexpr size_t smem = sizeof(FaceSmem16<NB, NQF>) * W;
     static unsigned long long done = 0;
-    if (const int rc = opt_in(face_flux_mixed16<NB, NQF, W>, smem, done)) return rc;
+    if (const int rc = ensure_smem(face_flux_mixed16<NB, NQF, W>, smem, done)) return rc;
     return a.ngroups > 0 ? launch_early(face_flux_mixed16<NB, NQF, W>, std::min((a.ngroups + W - 1) / W, sms), W * 32, smem, s, a) : (int)DG_OK;
 }
 
@@ -82,7 +71,7 @@ int run_element(int sms, const Mixed16ElemArgs& a, cudaStream_t s) {
     constexpr int W = element_warps<NB, NQV>();
     constexpr size_t smem = ElemSizes16<NB, NQV>::tables + sizeof(ElemSmem16<NB, NQV>) * W;
     static unsigned long long done = 0;
-    if (const int rc = opt_in(element_mixed16<NB, NQV, W>, smem, done)) return rc;
+    if (const int rc = ensure_smem(element_mixed16<NB, NQV, W>, smem, done)) return rc;
     return a.ngroups > 0 ? launch_early(element_mixed16<NB, NQV, W>, std::min((a.ngroups + W - 1) / W, sms), W * 32, smem, s, a) : (int)DG_OK;
 }
 
@@ -92,7 +81,7 @@ int run_stage(int sms, const Mixed16FaceArgs& fa, const Mixed16ElemArgs& ea, con
     constexpr int W = warps16(NB <= 10 ? 12 : 8, warp, tables);
     constexpr size_t smem = tables + warp * W;
     static unsigned long long done = 0;
-    if (const int rc = opt_in(stage_persistent_mixed16<NB, NQV, NQF, W>, smem, done)) return rc;
+    if (const int rc = ensure_smem(stage_persistent_mixed16<NB, NQV, NQF, W>, smem, done)) return rc;
     stage_persistent_mixed16<NB, NQV, NQF, W><<<sms, W * 32, smem, s>>>(fa, ea, q);
     return cuda_status(cudaGetLastError());
 }

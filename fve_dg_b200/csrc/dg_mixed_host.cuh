@@ -386,19 +386,6 @@ inline MixedElemArgs elem_args(const MixedData& m, const double* U, const double
     return ea;
 }
 
-// Opt a kernel into `smem` bytes of dynamic shared memory once per device.
-template <class Kernel>
-inline int ensure_smem(Kernel k, size_t smem, unsigned long long& done_mask) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return DG_E_CUDA;
-    const unsigned long long bit = 1ull << (dev & 63);
-    if (done_mask & bit) return DG_OK;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return DG_E_CUDA;
-    done_mask |= bit;
-    return DG_OK;
-}
-
 inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 inline Mixed16FaceArgs face_args16(const MixedData& m, const double* U, int face_mask, int g0 = 0, int g1 = -1) {

@@ -6,17 +6,6 @@
 namespace fvedg {
 namespace {
 
-template <class Kernel>
-int opt_in(Kernel k, size_t smem, unsigned long long& done_mask) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return DG_E_CUDA;
-    const unsigned long long bit = 1ull << (dev & 63);
-    if (done_mask & bit) return DG_OK;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return DG_E_CUDA;
-    done_mask |= bit;
-    return DG_OK;
-}
-
 // Eight warps per SM at 255 registers a thread, twelve at P1.
 constexpr int most_warps(int nb) { return nb <= 4 ? 12 : 8; }
 
@@ -25,7 +14,7 @@ int run_face(int sms, const Visc8Args& a, cudaStream_t s) {
     constexpr int W = warps16(most_warps(NB), sizeof(FaceSmem8<NB>));
     constexpr size_t smem = sizeof(FaceSmem8<NB>) * W;
     static unsigned long long done = 0;
-    if (const int rc = opt_in(visc_face_rows8<NB, NQF, CONV, W>, smem, done)) return rc;
+    if (const int rc = ensure_smem(visc_face_rows8<NB, NQF, CONV, W>, smem, done)) return rc;
     return a.f.ngroups > 0 ? launch_early(visc_face_rows8<NB, NQF, CONV, W>, std::min(a.f.ngroups, sms), W * 32, smem, s, a) : (int)DG_OK;
 }
 
@@ -34,12 +23,11 @@ int run_element(int sms, const Visc8Args& a, cudaStream_t s) {
     constexpr int W = warps16(most_warps(NB), sizeof(ElemSmem8<NB>));
     constexpr size_t smem = sizeof(ElemSmem8<NB>) * W;
     static unsigned long long done = 0;
-    if (const int rc = opt_in(visc_element_rows8<NB, NQV, CONV, W>, smem, done)) return rc;
+    if (const int rc = ensure_smem(visc_element_rows8<NB, NQV, CONV, W>, smem, done)) return rc;
     return a.e.ngroups > 0 ? launch_early(visc_element_rows8<NB, NQV, CONV, W>, std::min(a.e.ngroups, sms), W * 32, smem, s, a) : (int)DG_OK;
 }
 
 }  // namespace
-
 
 int visc8_face(int order, int qv, int qf, int sms, const Visc8Args& a, bool conv, cudaStream_t s) {
 #define X(P, QV, QF, NB, NQV, NQF)                                                                          \
