@@ -45,7 +45,7 @@
 #include "dg_internal.h"
 #include "dg_kernels_fp64.cuh"
 #include "dg_launch.cuh"
-#include "dg_tma.cuh"
+#include "dg_slots.cuh"
 
 namespace fvedg {
 
@@ -812,11 +812,7 @@ __device__ __forceinline__ bool element_group_staged(const MixedElemArgs& a, int
         const double dt = a.dt_inst ? __ldg(a.dt_inst + __ldg(a.elem_inst + e)) : a.dt;
         sm.sDT[lane] = dt * __ldg(a.inv_detj + e);
     }
-    if (!mbar_wait_bounded(&st.bar, parity, kBulkSpinLimit)) {
-        if (lane == 0 && a.err) *static_cast<volatile int*>(a.err) = DG_E_WATCHDOG;
-        mbar_wait_bounded(&st.bar, parity, kBulkSpinLimit);  // copies in flight land before the warp leaves
-        return false;
-    }
+    if (!warp_landed(&st.bar, parity, a.err, lane)) return false;
     if (lane < 16) sm.sC0[lane] = lane < 5 * ne ? (float)st.U[lane / 5][lane % 5] : 0.f;
     if (a.volume && lane < 5 * ne) {  // row k of G(c_0) = detJ F(c_0) J^-T, FP64, one lane per (element, var)
         const int el = lane / 5, k = lane - 5 * el;

@@ -49,16 +49,23 @@ struct RowSlotsOf {
     }
 };
 
-// Waits for the warp's rows, a bounded number of polls; when they run out, records it, lets the copies in
-// flight land (bounded again) and returns false to the whole warp.
-__device__ __forceinline__ bool rows_landed(uint64_t& bar, unsigned& parity, int* err, int lane) {
-    bool ok = mbar_wait_bounded(&bar, parity, kBulkSpinLimit);
+// The whole warp waits for phase `parity` of its barrier, a bounded number of polls. If they run out for any lane,
+// that is recorded, the copies in flight are let in (bounded again) and every lane has false: a lane that saw them land in
+// the last poll goes no further than the others.
+__device__ __forceinline__ bool warp_landed(uint64_t* bar, unsigned parity, int* err, int lane) {
+    const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, kBulkSpinLimit));
     if (!ok) {
         if (lane == 0 && err) *static_cast<volatile int*>(err) = DG_E_WATCHDOG;
-        mbar_wait_bounded(&bar, parity, kBulkSpinLimit);
+        mbar_wait_bounded(bar, parity, kBulkSpinLimit);
     }
+    return ok;
+}
+
+// The same for the warp's rows, whose barrier is in its next phase afterwards.
+__device__ __forceinline__ bool rows_landed(uint64_t& bar, unsigned& parity, int* err, int lane) {
+    const bool ok = warp_landed(&bar, parity, err, lane);
     parity ^= 1u;
-    return __all_sync(0xffffffffu, ok);
+    return ok;
 }
 
 }  // namespace fvedg
