@@ -157,7 +157,7 @@ __device__ __forceinline__ bool face_group8(const Rows8FaceArgs& a, int gi, Face
     for (int k = 0; k < 5; ++k)
         #pragma unroll
         for (int mt = 0; mt < MT; ++mt) mom[k][mt][0] = mom[k][mt][1] = 0.0;
-    if (!rows_landed(bar, parity, a.err, lane)) return false;
+    if (!rows_landed(bar, parity, a.err)) return false;
     #pragma unroll 1
     for (int nt = 0; nt < NT; ++nt) {
         double L[5][2], R[5][2];
@@ -292,7 +292,7 @@ __device__ __forceinline__ bool element_group8(const Rows8ElemArgs& a, int gi, E
         #pragma unroll
         for (int j = 0; j < NJ; ++j) acc[k][j][0] = acc[k][j][1] = 0.0;
     const double* row = Slots::at(sm.rows, gid, a.U + e * B5);
-    if (!rows_landed(bar, parity, a.err, lane)) return false;
+    if (!rows_landed(bar, parity, a.err)) return false;
     if (a.with_volume) {
         const double gm1 = a.gamma - 1.0;
         if constexpr (SHORT) {

@@ -63,13 +63,13 @@ int main() {
             warp.emplace_back([&, lane] {
                 static uint64_t bar;
                 late = (mask >> lane) & 1;
-                ok[lane] = rows_landed(bar, parity[lane], &err, lane);
+                ok[lane] = rows_landed(bar, parity[lane], &err);
                 waited[lane] = waits;
             });
         for (auto& t : warp) t.join();
         pthread_barrier_destroy(&meet);
         for (int lane = 0; lane < 32; ++lane)
-            if (ok[lane] != (mask == 0) || parity[lane] != 1u || waited[lane] != (mask ? 2 : 1)) {
+            if (ok[lane] != (mask == 0) || parity[lane] != 1u || waited[lane] != ((mask >> lane) & 1 ? 2 : 1)) {
                 std::printf("mask %x lane %d: %d, %d waits\n", mask, lane, ok[lane], waited[lane]);
                 return 1;
             }
