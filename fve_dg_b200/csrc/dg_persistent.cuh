@@ -55,6 +55,9 @@ __host__ __device__ constexpr size_t persistent_warp_smem() {
 #ifndef FVEDG_PERSIST_MINB8
 #define FVEDG_PERSIST_MINB8 4
 #endif
+// Launched early (dg_launch.cuh): its group functions read the state with plain loads, for the two launches' sake, which
+// alone cost P4 2 % (3,072 cells, us a step: 456 with read-only loads, 466 with plain ones, 452 early). P1, 3,072 cells
+// 120 -> 111; P2 153 -> 143; P3, 1,296 cells 238 -> 207; P2, 10,368 cells 165 -> 163.
 template <int NB, int NQV, int NQF, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? FVEDG_PERSIST_MINB8 : 6)
     stage_persistent_mixed(MixedFaceArgs fa, MixedElemArgs ea, TileQueue Q) {
@@ -62,6 +65,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? FVEDG_PERSIST_MINB8 :
     __shared__ ElemTables<NB> tabs;
     __shared__ int4 s_tile;
     element_tables_init(tabs, ea.t.inv_mass);
+    await_previous();  // every index below comes from a tile, taken after it
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned char* wsm = smem_raw + persistent_warp_smem<NB, NQV, NQF>() * warp;
     for (;;) {
@@ -82,6 +86,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? FVEDG_PERSIST_MINB8 :
             __syncthreads();
         }
     }
+    release_next();
     if (threadIdx.x == 0) leave_queue(Q);
 }
 
@@ -219,9 +224,8 @@ inline int persistent_launch(MixedData& m, QueueState* q, const QueueSchedule& q
         done |= 1ull << (dev & 63);
     }
     const int bps = pp.max_blocks > 0 ? std::min(per_sm[dev & 63], pp.max_blocks) : per_sm[dev & 63];
-    kern<<<m.sms * bps, W * 32, smem, s>>>(face_args(m, U, face_mask),
-                                           elem_args(m, U, U0, out, mode, dt, a0, a1, with_volume), tile_queue(q, qs, pp));
-    return cuda_status(cudaGetLastError());
+    return launch_early(kern, m.sms * bps, W * 32, smem, s, face_args(m, U, face_mask),
+                        elem_args(m, U, U0, out, mode, dt, a0, a1, with_volume), tile_queue(q, qs, pp));
 }
 
 inline int persistent_kernel(MixedData& m, QueueState* q, const QueueSchedule& qs, const PersistentParams& pp,
