@@ -574,28 +574,16 @@ int launches_per_step(const dg_ctx* c) {
     return 6 + lim;
 }
 
-// After a synchronize: the status words of the kernels' bounded waits (DG_OK or DG_E_WATCHDOG), cleared. They lie in
-// mapped host memory: read by copies from the device they were 8 us of every stepping call.
-int check_status(dg_ctx* c) {
-    int rc = DG_OK;
-    for (int i = 0; i < kStatusWords; ++i) {
-        volatile int* word = c->status + i;
-        if (*word == DG_OK) continue;
-        *word = DG_OK;
-        rc = DG_E_WATCHDOG;
-    }
-    return rc;
-}
+// After a synchronize: what the kernels' bounded waits have to report.
+int check_status(dg_ctx* c) { return take_status(c->status); }
 
-// The same, and the word of the persistent queue.
+// The same, and the word of the persistent queue, cleared in the order of the launches.
 int check_queue(dg_ctx* c) {
-    int err = 0;
-    if (const int rc = check_status(c)) return rc;
-    if (!c->d_queue || c->cfg.schedule != 1) return DG_OK;
-    if (cudaMemcpy(&err, &c->d_queue->error, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return DG_E_CUDA;
-    if (err == DG_OK) return DG_OK;
-    cudaMemset(c->d_queue, 0, sizeof(QueueState));
-    return DG_E_WATCHDOG;
+    if (!c->d_queue || c->cfg.schedule != 1) return check_status(c);
+    return take_status(
+        c->status,
+        [&](int* error) { return cuda_ok(cudaMemcpy(error, &c->d_queue->error, sizeof(int), cudaMemcpyDeviceToHost)); },
+        [&] { return cuda_ok(cudaMemsetAsync(c->d_queue, 0, sizeof(QueueState), c->stream)); });
 }
 
 // copy between a host buffer with element stride `stride` and a packed device buffer

@@ -60,4 +60,29 @@ class StatusPages {
     Page* first_ = nullptr;
 };
 
+// After a synchronize: DG_OK, or DG_E_WATCHDOG if a bounded wait ran out; the words are cleared. They lie in mapped host
+// memory: read by copies from the device they were 8 us of every stepping call.
+inline int take_status(int* words) {
+    int rc = DG_OK;
+    for (int i = 0; i < kStatusWords; ++i) {
+        volatile int* word = words + i;
+        if (*word == DG_OK) continue;
+        *word = DG_OK;
+        rc = DG_E_WATCHDOG;
+    }
+    return rc;
+}
+
+// The same with a tile queue's own error, which `read` fetches and `clear` re-arms (DG_OK or their own failure). Either is
+// taken whatever the other says: nothing that this call reports is left for the next.
+template <class Read, class Clear>
+int take_status(int* words, Read&& read, Clear&& clear) {
+    const int rc = take_status(words);
+    int error = DG_OK;
+    if (const int failed = read(&error)) return failed;
+    if (error == DG_OK) return rc;
+    if (const int failed = clear()) return failed;
+    return DG_E_WATCHDOG;
+}
+
 }  // namespace fvedg
