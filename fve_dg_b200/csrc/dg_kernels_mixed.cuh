@@ -812,7 +812,7 @@ __device__ __forceinline__ bool element_group_staged(const MixedElemArgs& a, int
         const double dt = a.dt_inst ? __ldg(a.dt_inst + __ldg(a.elem_inst + e)) : a.dt;
         sm.sDT[lane] = dt * __ldg(a.inv_detj + e);
     }
-    if (!warp_landed(&st.bar, parity, a.err)) return false;
+    if (!warp_landed<true>(&st.bar, parity, a.err)) return false;
     if (lane < 16) sm.sC0[lane] = lane < 5 * ne ? (float)st.U[lane / 5][lane % 5] : 0.f;
     if (a.volume && lane < 5 * ne) {  // row k of G(c_0) = detJ F(c_0) J^-T, FP64, one lane per (element, var)
         const int el = lane / 5, k = lane - 5 * el;

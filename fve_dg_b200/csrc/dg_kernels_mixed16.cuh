@@ -247,11 +247,11 @@ __device__ __forceinline__ bool face_group16(const Mixed16FaceArgs& a, int gi, i
             a.rec[(int64_t)grp.f[r] * RW + (i - r * RW)] = 0u;
         }
         // the rows in flight for it are let in, and the next group's sent for
-        if (!rows_landed(bar, parity, a.err)) return false;
+        if (!rows_landed<true>(bar, parity, a.err)) return false;
         if (next >= 0) Slots::load(sm.rows, lane, kRows, a.U + (int64_t)a.fi[a.groups[next].f[lane & 15]].c0 * (5 * NB), &bar);
         return true;
     }
-    auto landed = [&] { return rows_landed(bar, parity, a.err); };
+    auto landed = [&] { return rows_landed<true>(bar, parity, a.err); };
     // lane i < 16 moves row i: its cells in this group and the next
     const FaceInfo& mine = a.fi[grp.f[lane & 15]];
     const int right = mine.c1, more = next >= 0 ? a.groups[next].f[lane & 15] : -1;
@@ -551,7 +551,7 @@ __device__ __forceinline__ bool element_group16(const Mixed16ElemArgs& a, const 
     const ElemGroup16& grp = sm.grp[turn];
     const int n = grp.n;
     const bool u0 = a.mode != 0 && a.a0 != 0.0;
-    auto landed = [&] { return rows_landed(bar, parity, a.err); };
+    auto landed = [&] { return rows_landed<true>(bar, parity, a.err); };
     const int64_t mine = grp.e[lane & 15];  // lane i < 16 moves row i
     const bool more = next >= 0;
     if (more) elem_record16(a, next, sm.grp[turn ^ 1], lane);

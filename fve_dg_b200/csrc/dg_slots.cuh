@@ -49,21 +49,27 @@ struct RowSlotsOf {
     }
 };
 
-// The whole warp waits for phase `parity` of its barrier, a bounded number of polls. A lane whose polls run out records it
-// and lets the copies in flight land (bounded again); then every lane has false, also one that saw them land in its last
-// poll. (The vote is after the branch: before it, with a branch on its result, a P2 residual of 13,182 cells took 33.0 us, not 32.5.)
+// The whole warp waits for phase `parity` of its barrier, a bounded number of polls. If they run out for any lane, that is
+// recorded, the copies in flight are let in (bounded again) and every lane has false, also one that saw them land in its
+// last poll. The vote comes before the branch or after it, whichever the kernel is faster with (us, after / before): groups
+// of sixteen P2, four steps of 196,608 cells 2,856 / 2,816, P4, 93,750 cells 5,292 / 5,247, the persistent form 5,665 / 5,572;
+// the viscous kernels, a Navier-Stokes step at P3, 82,944 cells 1,931 / 1,922. But groups of eight, a residual, P2, 13,182 cells 32.7 / 33.0, P5, 7,986 cells 220 / 227.
+template <bool VOTE_FIRST>
 __device__ __forceinline__ bool warp_landed(uint64_t* bar, unsigned parity, int* err) {
-    const bool ok = mbar_wait_bounded(bar, parity, kBulkSpinLimit);
+    bool ok = mbar_wait_bounded(bar, parity, kBulkSpinLimit);
+    if constexpr (VOTE_FIRST) ok = __all_sync(0xffffffffu, ok);
     if (!ok) {
         if (err) *static_cast<volatile int*>(err) = DG_E_WATCHDOG;
         mbar_wait_bounded(bar, parity, kBulkSpinLimit);
     }
-    return __all_sync(0xffffffffu, ok);
+    if constexpr (!VOTE_FIRST) ok = __all_sync(0xffffffffu, ok);
+    return ok;
 }
 
 // The same for the warp's rows, whose barrier is in its next phase afterwards.
+template <bool VOTE_FIRST = false>
 __device__ __forceinline__ bool rows_landed(uint64_t& bar, unsigned& parity, int* err) {
-    const bool ok = warp_landed(&bar, parity, err);
+    const bool ok = warp_landed<VOTE_FIRST>(&bar, parity, err);
     parity ^= 1u;
     return ok;
 }

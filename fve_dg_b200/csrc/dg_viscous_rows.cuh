@@ -151,7 +151,7 @@ __device__ __forceinline__ bool visc_face_group8(const Visc8Args& A, int gi, Fac
     for (int k = 0; k < 6; ++k)
         #pragma unroll
         for (int mt = 0; mt < MT; ++mt) mom[k][mt][0] = mom[k][mt][1] = 0.0;
-    if (!rows_landed(bar, parity, a.err)) return false;
+    if (!rows_landed<true>(bar, parity, a.err)) return false;
     #pragma unroll 1
     for (int nt = 0; nt < NT; ++nt) {
         double V[2][5][2], X[2][5][3];  // [point]: averaged (boundary: inner) physical gradient
@@ -316,7 +316,7 @@ __device__ __forceinline__ bool visc_element_group8(const Visc8Args& A, int gi, 
         #pragma unroll
         for (int j = 0; j < NJ; ++j) acc[k][j][0] = acc[k][j][1] = 0.0;
     const double* row = Slots::at(sm.rows, gid, a.U + e * B5);
-    if (!rows_landed(bar, parity, a.err)) return false;
+    if (!rows_landed<true>(bar, parity, a.err)) return false;
     const double gm1 = a.gamma - 1.0;
     #pragma unroll 1
     for (int nt = 0; nt < NT; ++nt) {

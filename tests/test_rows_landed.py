@@ -48,7 +48,8 @@ bool __all_sync(unsigned, bool v) {
 namespace fvedg {
 bool mbar_wait_bounded(uint64_t*, unsigned, long long) { return ++waits > 1 || !late; }
 }
-int main() {
+template <bool VOTE_FIRST>
+int check() {
     // which lanes are late: none, one that is not lane 0, lane 0, all but lane 0, all
     const unsigned cases[] = {0u, 1u << 5, 1u, ~1u, ~0u};
     for (unsigned mask : cases) {
@@ -63,13 +64,13 @@ int main() {
             warp.emplace_back([&, lane] {
                 static uint64_t bar;
                 late = (mask >> lane) & 1;
-                ok[lane] = rows_landed(bar, parity[lane], &err);
+                ok[lane] = rows_landed<VOTE_FIRST>(bar, parity[lane], &err);
                 waited[lane] = waits;
             });
         for (auto& t : warp) t.join();
         pthread_barrier_destroy(&meet);
         for (int lane = 0; lane < 32; ++lane)
-            if (ok[lane] != (mask == 0) || parity[lane] != 1u || waited[lane] != ((mask >> lane) & 1 ? 2 : 1)) {
+            if (ok[lane] != (mask == 0) || parity[lane] != 1u || waited[lane] != ((VOTE_FIRST ? mask : (mask >> lane) & 1) ? 2 : 1)) {
                 std::printf("mask %x lane %d: %d, %d waits\n", mask, lane, ok[lane], waited[lane]);
                 return 1;
             }
@@ -77,6 +78,7 @@ int main() {
     }
     return 0;
 }
+int main() { const int rc = check<false>(); return rc ? rc : check<true>(); }
 """
 
 
