@@ -45,7 +45,7 @@ inline int rows8_upload(Rows8Data& m, const T** dst, const std::vector<T>& v) {
 }
 
 // Whether the convective operator of a mesh of that many cells runs in rows of eight. Orders 0 and 5 have no other
-// tensor-core kernels and take them at any size (P0 56 -> 39 us a step at n = 4 against the runtime-size kernels, P5
+// tensor-core kernels and take them at any size, if the groups are full enough (rows8_groups; P0 56 -> 39 us a step at n = 4 against the runtime-size kernels, P5
 // 326 -> 233; n = 24: 372 -> 260 and 16,345 -> 4,838). For the others groups of three are the faster on small meshes,
 // where a warp's chain of work decides (us a step, three / eight: P1 31 / 36 at n = 8, 34 / 36 at n = 9, 42 / 40 at
 // n = 11; P2 54 / 54 at n = 6, 60 / 56 at n = 8, 64 / 58 at n = 9; P3 68 / 74, 80 / 79, 93 / 81; P4 103 / 127, 131 / 134,

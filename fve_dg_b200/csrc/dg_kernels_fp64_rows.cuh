@@ -102,7 +102,7 @@ using Slots8 = RowSlotsOf<NB, slot_stride8((40 * NB + 8 + 15) / 16 * 16)>;
 // size of what is there already: residuals were 5 to 12 % further from the exact ones than those of the scalar kernels.
 // There the volume term is taken of the deviations from the mean state's flux (its own integral is one product), and
 // the sums of a point tile's moments and of a face are formed by themselves: 8 to 17 % closer than the scalar kernels,
-// 0.199 -> 0.215 ms a residual at 7,986 cells (scalar 0.521).
+// 0.203 -> 0.220 ms a residual at 7,986 cells (scalar 0.585).
 __host__ __device__ constexpr bool short_sums8(int nb) { return nb > 35; }
 
 // The five variables at the points 8 nt + 2 tq + {0, 1} of the lane's row: v[k] += sum_b c_b phi_b, with the row

@@ -31,7 +31,7 @@
 
 namespace fvedg {
 
-// Up to P1 the kernels are launched early (dg_launch.cuh; a step of 3,072 cells 35.0 -> 31.1 us). From P2 on what
+// Up to P1 the kernels are launched early (dg_launch.cuh; a step of 3,072 cells 35.7 -> 34.1 us). From P2 on what
 // that saves is lost on their loads, which then can't take the read-only path (P2 at 384 cells 49.5 -> 51.7 us, P4 94.6
 // -> 101).
 __host__ __device__ constexpr bool early_tc(int nb) { return nb <= 4; }

@@ -22,7 +22,7 @@ __device__ __forceinline__ int await_previous() {
 // the start, waiting blocks' shared memory took L1 from the running ones (mixed P4, 24,576 cells: 439 -> 493 us), and
 // blocks of which an SM holds several gathered on the few SMs that had room (FP64 P2, 1,296 cells: 54 -> 94 us).
 // So kernels with one block per SM call it as a warp begins its last item (FP64 P2, 7,986 cells: 74 -> 68 us), the
-// others at a warp's end (FP64 P1, 3,072 cells: 35 -> 31 us).
+// others at a warp's end (FP64 P1, 3,072 cells: 35.7 -> 34.1 us).
 __device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // A load of what an earlier kernel wrote and this one has not: free to move like one of constant memory, up to its
